@@ -26,6 +26,7 @@
 
 #include "ys_mas.cuh"
 #include "ys_mas_dev.cuh"
+#include "ys_mas_loop.cuh"
 
 namespace ys {
 
@@ -847,6 +848,133 @@ cudaError_t mas_add_update_nodes(void* mas, cudaGraph_t body, const cudaGraphNod
   }
   *last = n2;
   return e;
+}
+
+// Variables up to which the loop runs as one kernel (mas_pcg_loop): 24 us an
+// iteration against 34 for the graph of kernels at 31,744 variables (FEM cube,
+// FP32), 58 against 64 at 108,288, where the sixteen warps an SM no longer hide
+// the latency of data that comes from HBM.
+constexpr uint32_t kLoopMaxVars = 110000;
+
+template <typename T, bool WIDE>
+static cudaError_t add_loop_kernel(cudaGraph_t body, cudaGraphNode_t* node, LoopParams& L, uint32_t nv, int sms,
+                                   bool* used) {
+  int dev = 0, per_sm = 0, smem_max = 0;
+  const void* fn = (const void*)mas_pcg_loop<T, WIDE>;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  cudaFuncAttributes fa{};
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, fn);
+  if (e != cudaSuccess) return e;
+  const size_t area = 16ull * L.area, room = (size_t)smem_max - fa.sharedSizeBytes - 1024;
+  L.gemv_warps = (uint32_t)std::min<size_t>(kLoopThreads / 32, room / area);
+  if (L.gemv_warps == 0) return cudaSuccess;
+  const size_t smem = WIDE ? 2 * area : area * L.gemv_warps;  // the wide form: one area of doubles
+  e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kLoopThreads, smem);
+  if (e != cudaSuccess || per_sm < 1) return e;
+  // 64 rows a pass of a CTA; the wide form a domain a CTA (tiny systems take
+  // fewer CTAs: cheaper barriers)
+  const unsigned want = std::max(grid_for(nv, kLoopThreads / 4), WIDE ? L.M.num_domains : 1u);
+  const unsigned grid = std::min<unsigned>(want, (unsigned)sms);
+  void* args[] = {&L};
+  e = add_kernel(body, node, nullptr, 0, fn, grid, kLoopThreads, smem, args);
+  cudaKernelNodeAttrValue cv{};
+  cv.cooperative = 1;
+  if (e == cudaSuccess) e = cudaGraphKernelNodeSetAttribute(*node, cudaKernelNodeAttributeCooperative, &cv);
+  *used = e == cudaSuccess;
+  return e;
+}
+
+// The loop's own device memory: the segments of the rows longer than kLongRow
+// (from the row pointers), the grid's partial sums (a CTA an SM at most, more
+// than the workspace of a tiny system holds) and the wide form's corrections.
+static cudaError_t loop_memory(LoopParams& L, uint32_t nv, bool wide, unsigned max_grid, void** owned) {
+  std::vector<std::vector<uint32_t>> rp(L.nsets, std::vector<uint32_t>(nv + 1));
+  for (int s = 0; s < L.nsets; ++s) {
+    const cudaError_t e =
+        cudaMemcpy(rp[s].data(), L.sets[s].row_ptr, sizeof(uint32_t) * (nv + 1), cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) return e;
+  }
+  std::vector<uint4> seg;
+  std::vector<uint32_t> row, first;
+  for (uint32_t i = 0; i < nv; ++i) {
+    const size_t before = seg.size();
+    for (int s = 0; s < L.nsets; ++s) {
+      const uint32_t e0 = rp[s][i], e1 = rp[s][i + 1];
+      if (e1 - e0 <= kLongRow) continue;
+      for (uint32_t e = e0; e < e1; e += kLongSegment)
+        seg.push_back(make_uint4(i, e, std::min(e1, e + kLongSegment), (uint32_t)s));
+    }
+    if (seg.size() > before) {
+      row.push_back(i);
+      first.push_back((uint32_t)before);
+    }
+  }
+  L.num_segments = (uint32_t)seg.size();
+  L.num_long = (uint32_t)row.size();
+  first.push_back(L.num_segments);
+  const size_t b0 = sizeof(uint4) * seg.size(), b1 = sizeof(double) * 3 * seg.size();
+  const size_t b2 = sizeof(uint32_t) * row.size(), b3 = sizeof(uint32_t) * first.size();
+  const size_t bz = wide ? sizeof(double) * 3 * L.M.packed_nodes : 0;
+  const size_t bp = sizeof(double) * 3 * max_grid;  // p.q, r.z and r.r of every CTA
+  char* dev = nullptr;
+  cudaError_t e = cudaMalloc(&dev, bp + bz + 16 + b0 + b1 + b2 + b3);
+  if (e != cudaSuccess) return e;
+  *owned = dev;
+  L.partials = reinterpret_cast<double*>(dev);
+  L.zl64 = reinterpret_cast<double*>(dev + bp);
+  dev += (bp + bz + 15) / 16 * 16;
+  L.segments = reinterpret_cast<const uint4*>(dev);
+  L.seg = reinterpret_cast<double*>(dev + b0);
+  L.long_row = reinterpret_cast<const uint32_t*>(dev + b0 + b1);
+  L.long_first = reinterpret_cast<const uint32_t*>(dev + b0 + b1 + b2);
+  if (b0) e = cudaMemcpy(dev, seg.data(), b0, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && b2) e = cudaMemcpy(dev + b0 + b1, row.data(), b2, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(dev + b0 + b1 + b2, first.data(), b3, cudaMemcpyHostToDevice);
+  return e;
+}
+
+cudaError_t mas_add_loop_node(void* mas, cudaGraph_t body, MasPcgHooks* hooks, bool* used) {
+  *used = false;
+  auto* h = static_cast<MasHandle*>(mas);
+  auto* P = static_cast<MasPcg*>(hooks->params);
+  const MasDev& M = h->M;
+  if (P->nv > kLoopMaxVars) return cudaSuccess;
+  if (M.levels > 2 && M.packed_nodes - M.level_node_offset[2] > kLoopCoarse) return cudaSuccess;
+  LoopParams L{};
+  for (int s = 0; s < P->nsets; ++s) L.sets[s] = P->sets[s];
+  L.nsets = P->nsets;
+  L.M = M;
+  std::vector<uint32_t> ptr(M.num_domains + 1);
+  cudaError_t e = cudaMemcpy(ptr.data(), M.dom_node_ptr, sizeof(uint32_t) * ptr.size(), cudaMemcpyDeviceToHost);
+  if (e != cudaSuccess) return e;
+  for (uint32_t l = 0; l <= M.levels; ++l)
+    L.level_domain[l] = (uint32_t)(std::lower_bound(ptr.begin(), ptr.end(), M.level_node_offset[l]) - ptr.begin());
+  L.x = P->x;
+  L.r = P->r;
+  L.p = P->p;
+  L.p32 = P->p32;
+  L.q = P->q;
+  L.st = P->st;
+  L.arrivals = reinterpret_cast<unsigned long long*>(P->tickets + 4);
+  L.stop_rule = P->stop_rule;
+  L.area = (uint32_t)(gemv_smem_bytes(M.max_dofs) / 16);
+  L.cond = P->cond;
+  int dev = 0, sms = 0, coop = 0;
+  e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess || !coop) return e;
+  const bool wide = M.num_domains <= (uint32_t)sms;
+  e = loop_memory(L, P->nv, wide, (unsigned)sms, &hooks->owned);
+  cudaGraphNode_t node = nullptr;
+  if (e != cudaSuccess) return e;
+  if (wide)
+    return P->fp32 ? add_loop_kernel<float, true>(body, &node, L, P->nv, sms, used)
+                   : add_loop_kernel<double, true>(body, &node, L, P->nv, sms, used);
+  return P->fp32 ? add_loop_kernel<float, false>(body, &node, L, P->nv, sms, used)
+                 : add_loop_kernel<double, false>(body, &node, L, P->nv, sms, used);
 }
 
 }  // namespace ys

@@ -8,6 +8,7 @@ namespace ys {
 struct MasPcgHooks {
   void* params = nullptr;  // owned by the MAS handle
   bool fused_direction = false;  // the loop body's last MAS node also updates p
+  void* owned = nullptr;         // device memory of mas_add_loop_node (freed with the PCG handle)
 };
 
 // Nodes computing r = g - H x (or r = g), z = M^-1 r, p = z and the initial
@@ -23,5 +24,9 @@ cudaError_t mas_add_init_nodes(void* mas, cudaGraph_t g, const cudaGraphNode_t* 
 // beta and the stop test.
 cudaError_t mas_add_update_nodes(void* mas, cudaGraph_t body, const cudaGraphNode_t* deps, size_t ndeps,
                                  cudaGraphNode_t* last, MasPcgHooks* hooks);
+
+// The whole loop as one cooperative kernel, the body's only node, when the
+// system is small enough for it (*used).
+cudaError_t mas_add_loop_node(void* mas, cudaGraph_t body, MasPcgHooks* hooks, bool* used);
 
 }  // namespace ys

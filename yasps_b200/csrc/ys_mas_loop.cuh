@@ -1,0 +1,820 @@
+// The MAS-PCG iterations of a small or medium system in one cooperative
+// kernel (ys_mas.cu adds it as the body of the solve's conditional node).
+//
+// A graph of five to seven kernels an iteration costs its launches and the
+// tails of grids that are far too small for the chip, where the data of an
+// iteration sits in the 126 MB L2.  Here a resident grid (one CTA of 512
+// threads an SM, fewer for tiny systems) runs every iteration itself, with
+// four grid barriers:
+//   A  q = H p, p.q                       | barrier, every CTA sums the partials
+//   B  x += alpha p, r -= alpha q, r.r, level-1 residuals      | barrier
+//   C  z_d = A_d^-1 r_d for the domains of all levels, r.z     | barrier + sums
+//   D  z = sum_l w_l z_l, p = z + beta p                       | barrier
+// r.z is summed domain by domain, r.z = sum_l w_l (R_l r).z_l in FP64, so the
+// stop test and beta need no pass over z.  Loads that do not wait for a
+// barrier's result (row plans, the first tiles of an inverse) are issued
+// before it, those that do not wait for the sums before the sums.  Every CTA
+// forms the scalars from the same partials in the same order, so all take the
+// same decisions; the sums have a fixed order (deterministic).
+//
+// The wide form, for systems with at most a domain a CTA, applies the FP32
+// inverses with FP64 residuals, sums and corrections: the preconditioner is
+// then one fixed linear map.  On small ill-conditioned contact systems, where
+// the FP32 rounding of r and z was what the iteration fought with, it takes a
+// third to a sixth of the iterations (336 against 1862 on 70 vertices with
+// stiff friction), and a domain a CTA costs no more than in FP32.
+//
+// Barrier waits are bounded (kPollLimitParam polls): a CTA that gives up marks
+// the solve void (kBarrierFail) and every CTA leaves.
+#pragma once
+
+#include "ys_mas_dev.cuh"
+#include "ys_pcg.cuh"
+
+namespace ys {
+
+constexpr int kLoopThreads = 512;
+constexpr uint32_t kLoopCoarse = 512;    // most nodes of the levels from 2 on (their residuals in shared memory)
+constexpr uint32_t kLongRow = 64;        // longer rows are split over warps of the whole grid
+constexpr uint32_t kLongSegment = 128;   // entries a warp takes of a long row
+constexpr int kLoopMaxDofs = 4;          // 3-DoF entries a lane holds of a domain of at most 128 DoF
+
+struct LoopParams {
+  SpmvSet sets[2];
+  int nsets;
+  MasDev M;
+  uint32_t level_domain[kMaxLevels + 1];  // first domain of each level
+  double* x;
+  double* r;
+  double* p;
+  float4* p32;
+  double* q;
+  double* st;
+  double* partials;
+  unsigned long long* arrivals;
+  int stop_rule;
+  uint32_t gemv_warps;     // warps of a CTA with a GEMV area in shared memory
+  uint32_t area;           // float4 of one area
+  // long rows: segments (row, first entry, last entry, set) ordered by row and
+  // set; long_row lists the rows, long_first their first segments
+  const uint4* segments;
+  const uint32_t* long_row;
+  const uint32_t* long_first;
+  uint32_t num_segments, num_long;
+  double* seg;             // 3 per segment
+  double* zl64;            // the wide form's FP64 level corrections, 3 per packed node
+  cudaGraphConditionalHandle cond;
+};
+
+// Values other CTAs write in this kernel are read by plain loads (never the
+// read-only path); the barrier's acquire makes them current.
+__device__ __forceinline__ void loop_x(const float4* x, uint32_t j, float (&v)[3]) {
+  const float4 t = x[j];
+  v[0] = t.x; v[1] = t.y; v[2] = t.z;
+}
+__device__ __forceinline__ void loop_x(const double* x, uint32_t j, double (&v)[3]) {
+  v[0] = x[3ull * j]; v[1] = x[3ull * j + 1]; v[2] = x[3ull * j + 2];
+}
+
+template <typename T>
+struct LoopTypes;
+template <>
+struct LoopTypes<float> {
+  using X = float4;
+};
+template <>
+struct LoopTypes<double> {
+  using X = double;
+};
+
+__device__ __forceinline__ const float* set_values(const SpmvSet& s, float) { return s.values32; }
+__device__ __forceinline__ const double* set_values(const SpmvSet& s, double) { return s.values; }
+
+// State of the iteration, the same in every CTA; thread 0 writes it, the
+// others read it after the next CTA barrier.
+struct LoopState {
+  double delta, prev, rr, curv, alpha, beta, it;
+  unsigned long long target;
+  int status, ok;
+};
+
+// Bounded grid barrier on a monotonic arrival count; false: gave up.
+__device__ __forceinline__ bool loop_barrier(const LoopParams& P, LoopState& S) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned long long target = S.target + gridDim.x;
+    S.target = target;
+    int good = 1;
+    unsigned long long c;
+    // release: the CTA's writes (ordered before by the barrier above) are
+    // visible to whoever sees the arrival
+    asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(P.arrivals) : "memory");
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(c) : "l"(P.arrivals) : "memory");
+    if (c < target) {
+      const double limit = P.st[kPollLimitParam];
+      double polls = 0.0;
+      volatile double* fail = P.st + kBarrierFail;
+      while (c < target) {
+        if (polls >= limit || (((uint32_t)polls & 63u) == 63u && *fail != 0.0)) {
+          good = 0;
+          *fail = 1.0;
+          break;
+        }
+        polls += 1.0;
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(c) : "l"(P.arrivals) : "memory");
+      }
+    }
+    S.ok = good;
+  }
+  __syncthreads();
+  return S.ok != 0;
+}
+
+// Total of the grid's partials, by every warp for itself (all lanes get it, the
+// same bits in every warp and CTA): no CTA barrier on the path.
+__device__ __forceinline__ double loop_total(const double* partials) {
+  double a = 0.0;
+  for (unsigned b = threadIdx.x & 31; b < gridDim.x; b += 32) a += partials[b];
+  return warp_sum(a);
+}
+
+// The long rows' segments, a warp each; returns the lane's share of p.q.
+template <typename T>
+__device__ __forceinline__ double loop_segments(const LoopParams& P, const typename LoopTypes<T>::X* px) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double dot = 0.0;
+  for (uint32_t s = warp * gridDim.x + blockIdx.x; s < P.num_segments; s += (kLoopThreads / 32) * gridDim.x) {
+    const uint4 it = __ldg(P.segments + s);
+    const SpmvSet& S = P.sets[it.w];
+    const T* vals = set_values(S, T(0));
+    T a0 = 0, a1 = 0, a2 = 0;
+#pragma unroll 2
+    for (uint32_t e = it.y + lane; e < it.z; e += 32) {
+      const uint32_t eb = __ldg(S.entry_block + e), j = __ldg(S.entry_col + e);
+      T b[9], xv[3];
+      loop_x(px, j, xv);
+      load_block(vals, eb & 0x7fffffffu, b);
+      block_mac(b, xv, (eb & 0x80000000u) != 0, a0, a1, a2);
+    }
+    a0 = warp_sum(a0);
+    a1 = warp_sum(a1);
+    a2 = warp_sum(a2);
+    if (lane == 0) {
+      P.seg[3ull * s] = (double)a0;
+      P.seg[3ull * s + 1] = (double)a1;
+      P.seg[3ull * s + 2] = (double)a2;
+      const double* p = P.p + 3ull * it.x;
+      dot += p[0] * (double)a0 + p[1] * (double)a1 + p[2] * (double)a2;
+    }
+  }
+  return dot;
+}
+
+// Eight lanes a row, U rows a group of lanes at a time (rows of the CTA's
+// contiguous range, so neighbours meet in L1), two entries a lane and row in
+// flight.  The row bounds and the first two entries' indices of a round are
+// loaded a round ahead (those of the first before the barrier that completes
+// p): what is left on the path from the barrier is the gather of p.
+template <typename T, int U>
+struct LoopRows {
+  uint32_t e0[U], e1[U];
+  uint32_t eb[U][2], col[U][2];
+
+  __device__ __forceinline__ void bounds(const LoopParams& P, uint32_t base, uint32_t r1) {
+    const SpmvSet& S = P.sets[0];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t i = base + u * (kLoopThreads / 8);
+      const bool valid = i < r1;
+      e0[u] = valid ? __ldg(S.row_ptr + i) : 0u;
+      e1[u] = valid ? __ldg(S.row_ptr + i + 1) : 0u;
+      if (e1[u] - e0[u] > kLongRow) e1[u] = e0[u];
+    }
+  }
+  __device__ __forceinline__ void indices(const LoopParams& P, int sub) {
+    const SpmvSet& S = P.sets[0];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const uint32_t e = e0[u] + sub + kRowLanes * m;
+        const uint32_t k = e < e1[u] ? e : 0u;  // entry 0 stands in (its product is dropped)
+        eb[u][m] = __ldg(S.entry_block + k);
+        col[u][m] = __ldg(S.entry_col + k);
+      }
+  }
+};
+
+// q = H p for this CTA's rows over one block set; returns the thread's share
+// of p.q.  R holds the first round's rows on entry and the first round's again
+// on exit.
+template <typename T, int U>
+__device__ __forceinline__ double loop_spmv(const LoopParams& P, const typename LoopTypes<T>::X* px,
+                                            LoopRows<T, U>& R, uint32_t first, uint32_t r1) {
+  constexpr uint32_t kRows = kLoopThreads / 8;
+  const int sub = threadIdx.x & 7;
+  const SpmvSet& S = P.sets[0];
+  const T* vals = set_values(S, T(0));
+  double dot = 0.0;
+  // every lane runs the same rounds (the shuffles need whole warps)
+  const uint32_t warp_first = first - ((threadIdx.x & 31) >> 3);
+  for (uint32_t wb = warp_first; wb < r1; wb += U * kRows) {
+    const uint32_t base = wb + ((threadIdx.x & 31) >> 3);
+    T a[U][3];
+    uint32_t e0[U], e1[U];
+    double pr[U][3];
+    {
+      T xv[U][2][3], b[U][2][9];
+      uint32_t tr[U][2];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          loop_x(px, R.col[u][m], xv[u][m]);
+          load_block(vals, R.eb[u][m] & 0x7fffffffu, b[u][m]);
+          tr[u][m] = R.eb[u][m] & 0x80000000u;
+        }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        e0[u] = R.e0[u];
+        e1[u] = R.e1[u];
+        const uint32_t i = base + u * kRows;
+        if (i < r1 && sub == 0)
+#pragma unroll
+          for (int k = 0; k < 3; ++k) pr[u][k] = P.p[3ull * i + k];
+      }
+      // the next round's rows (the first round's after the last)
+      const bool more = wb + U * kRows < r1;
+      R.bounds(P, more ? base + U * kRows : first, r1);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        a[u][0] = a[u][1] = a[u][2] = 0;
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          T t0 = a[u][0], t1 = a[u][1], t2 = a[u][2];
+          block_mac(b[u][m], xv[u][m], tr[u][m] != 0, t0, t1, t2);
+          if (e0[u] + sub + kRowLanes * m < e1[u]) {
+            a[u][0] = t0;
+            a[u][1] = t1;
+            a[u][2] = t2;
+          }
+        }
+      }
+    }
+    R.indices(P, sub);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      for (uint32_t e = e0[u] + sub + 2 * kRowLanes; e < e1[u]; e += kRowLanes) {
+        const uint32_t eb = __ldg(S.entry_block + e), j = __ldg(S.entry_col + e);
+        T b[9], xv[3];
+        loop_x(px, j, xv);
+        load_block(vals, eb & 0x7fffffffu, b);
+        block_mac(b, xv, (eb & 0x80000000u) != 0, a[u][0], a[u][1], a[u][2]);
+      }
+#pragma unroll
+      for (int o = kRowLanes / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) a[u][k] += __shfl_xor_sync(0xffffffffu, a[u][k], o, kRowLanes);
+      const uint32_t i = base + u * kRows;
+      if (i < r1 && sub == 0) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          P.q[3ull * i + k] = (double)a[u][k];
+          dot += pr[u][k] * (double)a[u][k];
+        }
+      }
+    }
+  }
+  return dot;
+}
+
+// The same over two block sets (a static and a dynamic one), a row at a time.
+template <typename T>
+__device__ __forceinline__ double loop_spmv_sets(const LoopParams& P, const typename LoopTypes<T>::X* px,
+                                                 uint32_t first, uint32_t r1) {
+  const int sub = threadIdx.x & 7;
+  double dot = 0.0;
+  const uint32_t in_warp = (threadIdx.x & 31) >> 3;
+  for (uint32_t wb = first - in_warp; wb < r1; wb += kLoopThreads / 8) {
+    const uint32_t i = wb + in_warp;
+    const bool valid = i < r1;
+    double q[3] = {0.0, 0.0, 0.0};
+    for (int s = 0; s < P.nsets; ++s) {
+      const SpmvSet& S = P.sets[s];
+      const T* vals = set_values(S, T(0));
+      const uint32_t e0 = valid ? __ldg(S.row_ptr + i) : 0u, end = valid ? __ldg(S.row_ptr + i + 1) : 0u;
+      const uint32_t e1 = end - e0 > kLongRow ? e0 : end;
+      T a[3] = {0, 0, 0};
+      for (uint32_t e = e0 + sub; e < e1; e += kRowLanes) {
+        const uint32_t eb = __ldg(S.entry_block + e), j = __ldg(S.entry_col + e);
+        T b[9], xv[3];
+        loop_x(px, j, xv);
+        load_block(vals, eb & 0x7fffffffu, b);
+        block_mac(b, xv, (eb & 0x80000000u) != 0, a[0], a[1], a[2]);
+      }
+#pragma unroll
+      for (int o = kRowLanes / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) a[k] += __shfl_xor_sync(0xffffffffu, a[k], o, kRowLanes);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) q[k] += (double)a[k];
+    }
+    if (valid && sub == 0) {
+      const double* p = P.p + 3ull * i;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        P.q[3ull * i + k] = q[k];
+        dot += p[k] * q[k];
+      }
+    }
+  }
+  return dot;
+}
+
+// x += alpha p, r -= alpha q for a fine variable, in two parts: the loads do
+// not wait for alpha.
+struct LoopUpdate {
+  double q[3], p[3], x[3], r[3];
+  __device__ __forceinline__ void load(const LoopParams& P, uint32_t i) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      q[k] = P.q[3ull * i + k];
+      p[k] = P.p[3ull * i + k];
+      x[k] = P.x[3ull * i + k];
+      r[k] = P.r[3ull * i + k];
+    }
+    if (P.num_long) {
+      bool is_long = false;
+      for (int s = 0; s < P.nsets; ++s)
+        is_long |= __ldg(P.sets[s].row_ptr + i + 1) - __ldg(P.sets[s].row_ptr + i) > kLongRow;
+      if (is_long) {
+        uint32_t lo = 0, hi = P.num_long;  // long_row is ascending
+        while (hi - lo > 1) {
+          const uint32_t mid = (lo + hi) / 2;
+          if (__ldg(P.long_row + mid) <= i) lo = mid;
+          else hi = mid;
+        }
+        for (uint32_t s = __ldg(P.long_first + lo); s < __ldg(P.long_first + lo + 1); ++s)
+#pragma unroll
+          for (int k = 0; k < 3; ++k) q[k] += P.seg[3ull * s + k];
+      }
+    }
+  }
+  // the new residual is left in r; returns its squared norm
+  __device__ __forceinline__ double store(const LoopParams& P, uint32_t i, double alpha) {
+    double rr = 0.0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      P.x[3ull * i + k] = x[k] + p[k] * alpha;
+      r[k] = r[k] - q[k] * alpha;
+      P.r[3ull * i + k] = r[k];
+      rr += r[k] * r[k];
+    }
+    return rr;
+  }
+};
+
+// Residual sum of node p (packed id) over its children, by one warp (all
+// lanes get it); src holds the children's FP64 residuals, indexed by packed id
+// minus src_base.
+__device__ __forceinline__ void loop_child_sum(const MasDev& M, uint32_t p, const double* src, uint32_t src_base,
+                                               int lane, double (&s)[3]) {
+  const uint32_t c = p - M.nv;
+  s[0] = s[1] = s[2] = 0.0;
+  const uint32_t end = __ldg(M.child_ptr + c + 1);
+  for (uint32_t q = __ldg(M.child_ptr + c) + lane; q < end; q += 32) {
+    const double* v = src + 3ull * (__ldg(M.child_fine + q) - src_base);
+    s[0] += v[0];
+    s[1] += v[1];
+    s[2] += v[2];
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) s[k] = warp_sum(s[k]);
+}
+
+// Tiles of a domain's inverse a lane has in flight (3 and 4 spilled registers:
+// 27 and 29 us an iteration at 31,744 variables against 24).
+constexpr int kLoopTiles = 2;
+
+struct LoopTilesAhead {
+  float4 t[kLoopTiles][4];
+  __device__ __forceinline__ void load(const float4* src, int k, uint32_t slot, uint32_t tiles) {
+    if (slot < tiles) {
+#pragma unroll
+      for (int m = 0; m < 4; ++m) t[k][m] = __ldg(src + 4ull * slot + m);
+    }
+  }
+  // the first tiles of domain d (they do not wait for the residual)
+  __device__ __forceinline__ void first(const MasDev& M, uint32_t d) {
+    const uint32_t T = inv_tiles(3 * (__ldg(M.dom_node_ptr + d + 1) - __ldg(M.dom_node_ptr + d)));
+    const float4* src = reinterpret_cast<const float4*>(M.inverse + __ldg(M.inv_offset + d));
+#pragma unroll
+    for (int k = 0; k < kLoopTiles; ++k) load(src, k, (threadIdx.x & 31) + 32 * k, T * (T + 1) / 2);
+  }
+};
+
+// z_d = A_d^-1 r_d by one warp from its area of shared memory; `ahead` holds
+// the domain's first tiles, res the FP64 residuals of its level, indexed by
+// packed id minus res_base.  Returns the lane's share of w r_d . z_d.
+__device__ __forceinline__ double loop_gemv(const LoopParams& P, uint32_t d, LoopTilesAhead& ahead, const double* res,
+                                            uint32_t res_base, double w, float4* area) {
+  const MasDev& M = P.M;
+  const int lane = threadIdx.x & 31;
+  const uint32_t nb = __ldg(M.dom_node_ptr + d), n = 3 * (__ldg(M.dom_node_ptr + d + 1) - nb);
+  const uint32_t T = inv_tiles(n), ld = gemv_partial_ld(T), tiles = T * (T + 1) / 2;
+  const float4* src = reinterpret_cast<const float4*>(M.inverse + __ldg(M.inv_offset + d));
+  float4* part = area;
+  float* rloc = reinterpret_cast<float*>(area + T * ld);
+  double rv[kLoopMaxDofs];
+  uint32_t node[kLoopMaxDofs];
+#pragma unroll
+  for (int k = 0; k < kLoopMaxDofs; ++k) {
+    const uint32_t t = lane + 32 * k;
+    rv[k] = 0.0;
+    node[k] = 0;
+    if (t < n) {
+      node[k] = __ldg(M.dom_nodes + nb + t / 3);
+      rv[k] = res[3ull * (node[k] - res_base) + t % 3];
+    }
+    if (t < 4 * T) rloc[t] = (float)rv[k];
+  }
+  __syncwarp();
+  const float4* r4 = reinterpret_cast<const float4*>(rloc);
+  for (uint32_t s0 = lane; s0 < tiles; s0 += 32 * kLoopTiles) {
+#pragma unroll
+    for (int k = 0; k < kLoopTiles; ++k) {
+      const uint32_t slot = s0 + 32 * k;
+      if (slot < tiles) gemv_tile(T, ld, slot, ahead.t[k], r4, part);
+      ahead.load(src, k, slot + 32 * kLoopTiles, tiles);
+    }
+  }
+  __syncwarp();
+  double dot = 0.0;
+#pragma unroll
+  for (int k = 0; k < kLoopMaxDofs; ++k) {
+    const uint32_t i = lane + 32 * k;
+    if (i >= n) continue;
+    const float* row = reinterpret_cast<const float*>(part + (i / 4) * ld) + (i % 4);
+    float s0 = 0.0f, s1 = 0.0f;
+    for (uint32_t y = 0; y < T; y += 2) {  // T is even
+      s0 += row[4 * y];
+      s1 += row[4 * y + 4];
+    }
+    const float z = s0 + s1;
+    M.zl[3ull * node[k] + i % 3] = z;
+    dot += rv[k] * (double)z;
+  }
+  __syncwarp();
+  return w * dot;
+}
+
+// A tile's products in the CTA form: the same cells as gemv_tile, R the type
+// of the residual and of the sums.
+template <typename R>
+struct alignas(16) Quad {
+  R v[4];
+};
+template <typename R>
+__device__ __forceinline__ void loop_tile(uint32_t T, uint32_t ld, uint32_t slot, const float4 (&t)[4], const R* r,
+                                          Quad<R>* part) {
+  // see gemv_tile for the slot's (A, B)
+  const uint32_t q = (uint32_t)(((float)slot + 0.5f) * (1.0f / (float)(T + 1)));
+  const uint32_t c = slot - q * (T + 1);
+  const bool first = c < T - q;
+  const uint32_t A = first ? q : T - 1 - q;
+  const uint32_t B = first ? q + c : A + (c - (T - q));
+  const R m[4][4] = {{t[0].x, t[0].y, t[0].z, t[0].w},
+                     {t[1].x, t[1].y, t[1].z, t[1].w},
+                     {t[2].x, t[2].y, t[2].z, t[2].w},
+                     {t[3].x, t[3].y, t[3].z, t[3].w}};
+  Quad<R> x = *reinterpret_cast<const Quad<R>*>(r + 4 * B), u;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    u.v[i] = mac(m[i][3], x.v[3], mac(m[i][2], x.v[2], mac(m[i][1], x.v[1], m[i][0] * x.v[0])));
+  part[A * ld + B] = u;
+  if (A != B) {
+    x = *reinterpret_cast<const Quad<R>*>(r + 4 * A);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      u.v[i] = mac(m[3][i], x.v[3], mac(m[2][i], x.v[2], mac(m[1][i], x.v[1], m[0][i] * x.v[0])));
+    part[B * ld + A] = u;
+  }
+}
+
+// z_d = A_d^-1 r_d by the whole CTA, a tile a thread, the tiles prefetched
+// before the residuals are summed.
+template <typename R>
+__device__ __forceinline__ double loop_gemv_cta(const LoopParams& P, uint32_t d, const float4 (&tile)[4],
+                                                const double* res, uint32_t res_base, double w, float4* area, R* zl) {
+  const MasDev& M = P.M;
+  const uint32_t nb = __ldg(M.dom_node_ptr + d), n = 3 * (__ldg(M.dom_node_ptr + d + 1) - nb);
+  const uint32_t T = inv_tiles(n), ld = gemv_partial_ld(T), tiles = T * (T + 1) / 2;
+  Quad<R>* part = reinterpret_cast<Quad<R>*>(area);
+  R* rloc = reinterpret_cast<R*>(part + T * ld);
+  const uint32_t t = threadIdx.x;
+  double rv = 0.0;
+  uint32_t node = 0;
+  if (t < n) {
+    node = __ldg(M.dom_nodes + nb + t / 3);
+    rv = res[3ull * (node - res_base) + t % 3];
+  }
+  if (t < 4 * T) rloc[t] = (R)rv;
+  __syncthreads();
+  if (t < tiles) loop_tile<R>(T, ld, t, tile, rloc, part);
+  const float4* src = reinterpret_cast<const float4*>(M.inverse + __ldg(M.inv_offset + d));
+  for (uint32_t slot = t + kLoopThreads; slot < tiles; slot += kLoopThreads) {
+    float4 more[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) more[m] = __ldg(src + 4ull * slot + m);
+    loop_tile<R>(T, ld, slot, more, rloc, part);
+  }
+  __syncthreads();
+  double dot = 0.0;
+  if (t < n) {
+    const R* row = reinterpret_cast<const R*>(part + (t / 4) * ld) + (t % 4);
+    R s0 = 0, s1 = 0;
+    for (uint32_t y = 0; y < T; y += 2) {  // T is even
+      s0 += row[4 * y];
+      s1 += row[4 * y + 4];
+    }
+    const R z = s0 + s1;
+    zl[3ull * node + t % 3] = z;
+    dot = w * rv * (double)z;
+  }
+  __syncthreads();
+  return dot;
+}
+
+__device__ __forceinline__ void loop_prefetch(const MasDev& M, uint32_t d, float4 (&tile)[4]) {
+  const uint32_t T = inv_tiles(3 * (__ldg(M.dom_node_ptr + d + 1) - __ldg(M.dom_node_ptr + d)));
+  if (threadIdx.x < T * (T + 1) / 2) {
+    const float4* src = reinterpret_cast<const float4*>(M.inverse + __ldg(M.inv_offset + d)) + 4ull * threadIdx.x;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) tile[m] = __ldg(src + m);
+  }
+}
+
+// Residuals of the levels 2 .. l that domain d of level l needs, in `coarse`
+// (indexed by packed id minus the level-2 offset).
+__device__ __forceinline__ void loop_coarse(const LoopParams& P, uint32_t d, uint32_t l, double* coarse) {
+  const MasDev& M = P.M;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t l2 = M.level_node_offset[2];
+  const uint32_t nb = __ldg(M.dom_node_ptr + d), nn = __ldg(M.dom_node_ptr + d + 1) - nb;
+  for (uint32_t lev = 2; lev <= l; ++lev) {
+    const uint32_t base = M.level_node_offset[lev];
+    const uint32_t count = lev == l ? nn : M.level_node_offset[lev + 1] - base;
+    for (uint32_t c = warp; c < count; c += kLoopThreads / 32) {
+      const uint32_t p = lev == l ? __ldg(M.dom_nodes + nb + c) : base + c;
+      double s[3];
+      if (lev == 2) loop_child_sum(M, p, M.rl64, 0u, lane, s);
+      else loop_child_sum(M, p, coarse, l2, lane, s);
+      if (lane < 3) coarse[3 * (p - l2) + lane] = lane == 0 ? s[0] : (lane == 1 ? s[1] : s[2]);
+    }
+    __syncthreads();
+  }
+}
+
+// z_i = sum_l w_l z_l(map_l(i)).
+template <bool WIDE>
+__device__ __forceinline__ void loop_collect(const LoopParams& P, uint32_t i, double (&z)[3]) {
+  if constexpr (!WIDE) {
+    collect_levels(P.M, P.M.nv, i, z);
+  } else {
+    z[0] = z[1] = z[2] = 0.0;
+    for (uint32_t l = 0; l < P.M.levels; ++l) {
+      const double* v = P.zl64 + 3ull * __ldg(P.M.cmap + (uint64_t)l * P.M.nv + i);
+      const double w = (double)P.M.weight[l];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) z[k] += w * v[k];
+    }
+  }
+}
+
+template <typename T, bool WIDE>
+__global__ void __launch_bounds__(kLoopThreads, 1) mas_pcg_loop(const __grid_constant__ LoopParams P) {
+  extern __shared__ float4 loop_areas[];
+  __shared__ double red[kLoopThreads / 32];
+  __shared__ double coarse[3 * kLoopCoarse];
+  __shared__ LoopState S;
+  const MasDev& M = P.M;
+  double* const st = P.st;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kWarps = kLoopThreads / 32;
+  const typename LoopTypes<T>::X* px;
+  if constexpr (sizeof(T) == 4) px = P.p32;
+  else px = P.p;
+  if (threadIdx.x == 0) {
+    S.delta = st[kDeltaNew];
+    S.prev = S.delta;
+    S.rr = st[kRR];
+    S.it = st[kIter];
+    S.curv = S.alpha = S.beta = 0.0;
+    S.target = 0ull;
+    S.status = (int)st[kStatus];
+  }
+  // this CTA's rows
+  const uint32_t per = ((M.nv + gridDim.x - 1) / gridDim.x + 3u) & ~3u;
+  const uint32_t r1 = min(M.nv, (blockIdx.x + 1) * per);
+  const uint32_t first_row = blockIdx.x * per + (threadIdx.x >> 3);
+  constexpr int U = 1;  // 2 spilled registers: slower
+  LoopRows<T, U> rows;
+  if (P.nsets == 1) {
+    rows.bounds(P, first_row, r1);
+    rows.indices(P, threadIdx.x & 7);
+  }
+  __syncthreads();
+  while (S.status == kContinue) {
+    // A
+    {
+      double dot = P.nsets == 1 ? loop_spmv<T, U>(P, px, rows, first_row, r1)
+                                : loop_spmv_sets<T>(P, px, first_row, r1);
+      if (P.num_segments) dot += loop_segments<T>(P, px);
+      const double s = block_sum<kLoopThreads>(dot, red);
+      if (threadIdx.x == 0) P.partials[blockIdx.x] = s;
+    }
+    if (!loop_barrier(P, S)) break;
+    // the first variables of B are on their way while the step length is summed
+    LoopUpdate up;
+    uint32_t up_i = 0, up_p = 0, up_q = 0, up_end = 0;
+    bool up_on = false;
+    if (M.levels > 1) {
+      up_p = M.level_node_offset[1] + warp * gridDim.x + blockIdx.x;
+      if (up_p < M.level_node_offset[2]) {
+        up_end = __ldg(M.child_ptr + (up_p - M.nv) + 1);
+        up_q = __ldg(M.child_ptr + (up_p - M.nv)) + lane;
+        up_on = up_q < up_end;
+        if (up_on) up_i = __ldg(M.child_fine + up_q);
+      }
+    } else {
+      up_i = blockIdx.x * kLoopThreads + threadIdx.x;
+      up_on = up_i < M.nv;
+    }
+    if (up_on) up.load(P, up_i);
+    const double curv = loop_total(P.partials), prev = S.delta;
+    const bool restart = isfinite(curv) && curv <= 0.0 && isfinite(prev) && prev > 0.0;
+    if (!restart && (!isfinite(curv) || curv <= 0.0)) {
+      if (threadIdx.x == 0) {
+        S.curv = curv;
+        S.alpha = 0.0;
+        S.prev = prev;
+        S.it += 1.0;
+        S.status = kNonSpd;
+      }
+      break;
+    }
+    // (restart: finite non-positive curvature, zero step; see spmv_dot_finish)
+    const double alpha = restart ? 0.0 : prev / curv;
+    // B
+    double acc = 0.0;
+    {
+      if (M.levels > 1) {
+        for (; up_p < M.level_node_offset[2]; up_p += kWarps * gridDim.x) {  // warp-uniform
+          double s[3] = {0.0, 0.0, 0.0};
+          while (up_on) {
+            acc += up.store(P, up_i, alpha);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) s[k] += up.r[k];
+            up_q += 32;
+            up_on = up_q < up_end;
+            if (up_on) {
+              up_i = __ldg(M.child_fine + up_q);
+              up.load(P, up_i);
+            }
+          }
+#pragma unroll
+          for (int k = 0; k < 3; ++k) s[k] = warp_sum(s[k]);
+          if (lane < 3) M.rl64[3ull * up_p + lane] = lane == 0 ? s[0] : (lane == 1 ? s[1] : s[2]);
+          const uint32_t np = up_p + kWarps * gridDim.x;
+          if (np < M.level_node_offset[2]) {
+            up_end = __ldg(M.child_ptr + (np - M.nv) + 1);
+            up_q = __ldg(M.child_ptr + (np - M.nv)) + lane;
+            up_on = up_q < up_end;
+            if (up_on) {
+              up_i = __ldg(M.child_fine + up_q);
+              up.load(P, up_i);
+            }
+          }
+        }
+      } else {
+        while (up_on) {
+          acc += up.store(P, up_i, alpha);
+          up_i += gridDim.x * kLoopThreads;
+          up_on = up_i < M.nv;
+          if (up_on) up.load(P, up_i);
+        }
+      }
+      const double s = block_sum<kLoopThreads>(acc, red);
+      if (threadIdx.x == 0) P.partials[2 * gridDim.x + blockIdx.x] = s;
+    }
+    // the first tiles of the warp's (or CTA's) first domain are on their way
+    // over the barrier; the coarsest domains go to the first CTAs
+    const uint32_t first2 = M.levels > 2 ? P.level_domain[2] : M.num_domains;
+    const uint32_t first1 = M.levels > 1 ? P.level_domain[1] : M.num_domains, n1 = first2 - first1;
+    const uint32_t whole = WIDE ? M.num_domains : M.num_domains - first2;  // domains by whole CTAs, from the last
+    // the other CTAs share the rest, a warp a domain, when there are enough
+    const uint32_t skip = !WIDE && whole < gridDim.x / 2 ? whole : 0;
+    const uint32_t workers = gridDim.x - skip;
+    uint32_t job = first2;
+    if (!WIDE && warp < (int)P.gemv_warps && blockIdx.x >= skip) job = warp * workers + (blockIdx.x - skip);
+    LoopTilesAhead ahead;
+    if (blockIdx.x < whole) loop_prefetch(M, M.num_domains - 1 - blockIdx.x, ahead.t[0]);
+    else if (job < first2) ahead.first(M, job < n1 ? first1 + job : job - n1);
+    if (!loop_barrier(P, S)) break;
+    // C
+    acc = 0.0;
+    {
+      for (uint32_t k = blockIdx.x; k < whole; k += gridDim.x) {
+        const uint32_t d = M.num_domains - 1 - k;
+        uint32_t l = 0;
+        while (l + 1 < M.levels && d >= P.level_domain[l + 1]) ++l;
+        if (k != blockIdx.x) loop_prefetch(M, d, ahead.t[0]);
+        if (l >= 2) loop_coarse(P, d, l, coarse);
+        const double* res = l >= 2 ? coarse : (l == 1 ? M.rl64 : P.r);
+        const uint32_t base = l >= 2 ? M.level_node_offset[2] : 0u;
+        if constexpr (WIDE)
+          acc += loop_gemv_cta<double>(P, d, ahead.t[0], res, base, (double)M.weight[l], loop_areas, P.zl64);
+        else
+          acc += loop_gemv_cta<float>(P, d, ahead.t[0], res, base, (double)M.weight[l], loop_areas, M.zl);
+      }
+      if constexpr (!WIDE) {
+        float4* const area = loop_areas + (size_t)warp * P.area;
+        const bool fresh = blockIdx.x >= whole;  // `ahead` still holds the first job's tiles
+        for (uint32_t j = job; j < first2; j += P.gemv_warps * workers) {
+          const bool one = j < n1;  // the level-1 domains first
+          const uint32_t d = one ? first1 + j : j - n1;
+          if (j != job || !fresh) ahead.first(M, d);
+          acc += loop_gemv(P, d, ahead, one ? M.rl64 : P.r, 0u, (double)M.weight[one ? 1 : 0], area);
+        }
+      }
+      const double s = block_sum<kLoopThreads>(acc, red);
+      if (threadIdx.x == 0) P.partials[gridDim.x + blockIdx.x] = s;
+    }
+    if (!loop_barrier(P, S)) break;
+    // the first z of D while the totals are summed
+    double z[3] = {0.0, 0.0, 0.0}, pold[3] = {0.0, 0.0, 0.0};
+    const uint32_t d_i = blockIdx.x * kLoopThreads + threadIdx.x;
+    if (d_i < M.nv) {
+      loop_collect<WIDE>(P, d_i, z);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) pold[k] = P.p[3ull * d_i + k];
+    }
+    const double delta = loop_total(P.partials + gridDim.x), rr = loop_total(P.partials + 2 * gridDim.x);
+    double beta = 0.0;
+    int status = kContinue;
+    const double it = S.it + 1.0;
+    // mas/pcg.py:80-98
+    if (!isfinite(delta) || delta < 0.0 || !isfinite(prev) || prev <= 0.0) {
+      status = kNonSpd;
+    } else {
+      beta = restart ? 0.0 : delta / prev;
+      const bool done = P.stop_rule == YS_STOP_RESIDUAL ? rr <= st[kTolAbs] : delta <= st[kTolAbs];
+      if (done) status = kConverged;
+      else if (delta == 0.0) status = kNonSpd;
+      else if (it >= st[kMaxItParam]) status = kMaxIter;
+    }
+    __syncthreads();  // every warp has read S.it
+    if (threadIdx.x == 0) {
+      S.delta = delta;
+      S.prev = prev;
+      S.rr = rr;
+      S.curv = curv;
+      S.alpha = alpha;
+      S.beta = beta;
+      S.it = it;
+      S.status = status;
+    }
+    if (status != kContinue) break;
+    // D
+    {
+      for (uint32_t i = d_i; i < M.nv; i += gridDim.x * kLoopThreads) {
+        if (i != d_i) {
+          loop_collect<WIDE>(P, i, z);
+#pragma unroll
+          for (int k = 0; k < 3; ++k) pold[k] = P.p[3ull * i + k];
+        }
+        double p[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          p[k] = z[k] + pold[k] * beta;
+          P.p[3ull * i + k] = p[k];
+        }
+        if (sizeof(T) == 4) P.p32[i] = make_float4((float)p[0], (float)p[1], (float)p[2], 0.0f);
+      }
+    }
+    if (!loop_barrier(P, S)) break;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    st[kDeltaNew] = S.delta;
+    st[kDeltaOld] = S.prev;
+    st[kCurv] = S.curv;
+    st[kAlpha] = S.alpha;
+    st[kBeta] = S.beta;
+    st[kRR] = S.rr;
+    st[kIter] = S.it;
+    st[kStatus] = (double)S.status;
+    cudaGraphSetConditional(P.cond, 0u);
+  }
+}
+
+}  // namespace ys

@@ -604,7 +604,11 @@ int32_t ys_pcg_create(const ys_pcg_args* args, void** handle) {
       cudaGraph_t body = cp.conditional.phGraph_out[0];
       cudaGraphNode_t n1 = nullptr, n2 = nullptr, n3 = nullptr;
       void* args1[] = {&P};
-      if (streamed)
+      bool looped = false;
+      if (a.preconditioner == YS_PREC_MAS) e = ys::mas_add_loop_node(a.mas, body, &h->mas, &looped);
+      if (e != cudaSuccess || looped) {
+        // one kernel runs every iteration
+      } else if (streamed)
         e = ys::add_kernel(body, &n1, nullptr, 0, (const void*)ys::pcg_spmv_dot_streamed, grid_tiles,
                            ys::kTileThreads, args1, tile_smem);
       else if (tiled)
@@ -614,7 +618,7 @@ int32_t ys_pcg_create(const ys_pcg_args* args, void** handle) {
         e = ys::add_kernel(body, &n1, nullptr, 0,
                            P.fp32 ? (const void*)ys::pcg_spmv_dot<true> : (const void*)ys::pcg_spmv_dot<false>,
                            grid_rows, ys::kPcgBlock, args1);
-      if (e == cudaSuccess) {
+      if (e == cudaSuccess && !looped) {
         if (a.preconditioner == YS_PREC_BLOCK_JACOBI) {
           e = ys::add_kernel(body, &n2, &n1, 1,
                              P.jgroup ? (const void*)ys::pcg_update_bjw : (const void*)ys::pcg_update_bj, grid,
@@ -623,7 +627,7 @@ int32_t ys_pcg_create(const ys_pcg_args* args, void** handle) {
           e = ys::mas_add_update_nodes(a.mas, body, &n1, 1, &n2, &h->mas);
         }
       }
-      if (e == cudaSuccess && a.preconditioner != YS_PREC_BLOCK_JACOBI && h->mas.fused_direction)
+      if (looped || (e == cudaSuccess && a.preconditioner != YS_PREC_BLOCK_JACOBI && h->mas.fused_direction))
         n3 = n2;  // the MAS collect kernel updated p already
       else if (e == cudaSuccess)
         e = ys::add_kernel(body, &n3, &n2, 1, (const void*)ys::pcg_direction, grid, ys::kPcgBlock, args1);
@@ -636,6 +640,7 @@ int32_t ys_pcg_create(const ys_pcg_args* args, void** handle) {
     if (h->exec) cudaGraphExecDestroy(h->exec);
     if (h->graph) cudaGraphDestroy(h->graph);
     if (h->slots_host) cudaFreeHost(h->slots_host);
+    if (h->mas.owned) cudaFree(h->mas.owned);
     delete h;
     return YS_ERR_CUDA;
   }
@@ -758,6 +763,7 @@ int32_t ys_pcg_destroy(void* handle) {
   if (h->exec) cudaGraphExecDestroy(h->exec);
   if (h->graph) cudaGraphDestroy(h->graph);
   if (h->slots_host) cudaFreeHost(h->slots_host);
+  if (h->mas.owned) cudaFree(h->mas.owned);
   delete h;
   return YS_OK;
 }
