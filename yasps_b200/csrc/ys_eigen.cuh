@@ -18,12 +18,9 @@ namespace ys {
 __host__ __device__ constexpr int tri(int r, int c) { return r * (r + 1) / 2 + c; }
 
 // In-place test on a packed lower triangle `s` (destroyed).  Returns true when
-// the matrix is positive semidefinite within 1e-10 * max(1, max |A_ii|).
+// the matrix is positive semidefinite within 1e-10 * scale.
 template <int N>
-__device__ __forceinline__ bool psd_test_packed(double* s) {
-  double scale = 1.0;
-#pragma unroll
-  for (int r = 0; r < N; ++r) scale = fmax(scale, fabs(s[tri(r, r)]));
+__device__ __forceinline__ bool psd_test_packed(double* s, double scale) {
   const double tol = scale * 1.0e-10;
   bool ok = true;
 #pragma unroll
@@ -45,6 +42,41 @@ __device__ __forceinline__ bool psd_test_packed(double* s) {
     }
   }
   return ok;
+}
+
+// The same with the reference's scale, max(1, max |A_ii|).
+template <int N>
+__device__ __forceinline__ bool psd_test_packed(double* s) {
+  double scale = 1.0;
+#pragma unroll
+  for (int r = 0; r < N; ++r) scale = fmax(scale, fabs(s[tri(r, r)]));
+  return psd_test_packed<N>(s, scale);
+}
+
+// The same test of a translation-invariant 3A x 3A matrix from its leading
+// N = 3 (A - 1) rows (packed lower, destroyed) and the whole matrix's scale.
+// While no pivot is skipped, the last vertex's rows stay minus the sum of the
+// others, so its three pivots are rounding (below 1e-13 of the scale) and the
+// leading pivots decide: 1 PSD, 0 not.  A pivot within the tolerance gives -1:
+// the whole matrix has to be tested.
+template <int N>
+__device__ __forceinline__ int psd_test_leading(double* s, double scale) {
+  const double tol = scale * 1.0e-10;
+  bool neg = false, skip = false;
+#pragma unroll
+  for (int c = 0; c < N; ++c) {
+    const double pivot = s[tri(c, c)];
+    neg |= pivot < -tol && !skip;
+    skip |= fabs(pivot) <= tol;
+    const double inv = __drcp_rn(pivot);
+#pragma unroll
+    for (int r = c + 1; r < N; ++r) {
+      const double f = s[tri(r, c)] * inv;
+#pragma unroll
+      for (int t = c + 1; t <= r; ++t) s[tri(r, t)] = __fma_rn(-f, s[tri(t, c)], s[tri(r, t)]);
+    }
+  }
+  return neg ? 0 : (skip ? -1 : 1);
 }
 
 // Cyclic Jacobi on a full symmetric N x N matrix a (row-major, overwritten
@@ -170,15 +202,19 @@ __host__ __device__ constexpr int project_stash_doubles() {
   return N * (N + 1) / 2 + (N - 1) * N / 2 - 1 + (N - 2);
 }
 
-template <int N>
+// STASHED: the stash holds the matrix already (beside its copy in `a`), and
+// the result is left there only.
+template <int N, bool STASHED = false>
 __device__ __forceinline__ void project_negative_modes(double (&a)[N * (N + 1) / 2], int method,
                                                        double* __restrict__ stash, int stride) {
   constexpr int KS = N * (N + 1) / 2;        // original matrix
   constexpr int RS = KS;                     // reflector k, entries k+1..N-1
   constexpr int BS = RS + (N - 1) * N / 2 - 1;  // beta_k
   auto refl = [](int k, int i) { return k * (2 * N - k - 1) / 2 + (i - k - 1); };  // rows k = 0..N-3
+  if constexpr (!STASHED) {
 #pragma unroll
-  for (int i = 0; i < KS; ++i) stash[i * stride] = a[i];
+    for (int i = 0; i < KS; ++i) stash[i * stride] = a[i];
+  }
   // -- 1. tridiagonalisation ------------------------------------------------------
   double e[N];
 #pragma unroll
@@ -229,8 +265,10 @@ __device__ __forceinline__ void project_negative_modes(double (&a)[N * (N + 1) /
     g = fmax(g, r);
   }
   if (!(g > 0.0) || !isfinite(g)) {
+    if constexpr (!STASHED) {
 #pragma unroll
-    for (int i = 0; i < KS; ++i) a[i] = stash[i * stride];
+      for (int i = 0; i < KS; ++i) a[i] = stash[i * stride];
+    }
     return;
   }
   // unit scale (Gershgorin bound 1)
@@ -347,8 +385,10 @@ __device__ __forceinline__ void project_negative_modes(double (&a)[N * (N + 1) /
         for (int j = i; j < N; ++j) stash[utri<N>(i, j) * stride] += w * y[i] * y[j];
     }
   }
+  if constexpr (!STASHED) {
 #pragma unroll
-  for (int i = 0; i < KS; ++i) a[i] = stash[i * stride];
+    for (int i = 0; i < KS; ++i) a[i] = stash[i * stride];
+  }
 }
 
 }  // namespace ys

@@ -12,19 +12,19 @@
 //
 // Projection (the reference projects this full 12x12 matrix,
 // PKG/differentiator/differentiator.pyx:794-799, hessianKernelHeader.pyx:224-252):
-// the exact LDL^T PSD test runs on A; for the others, W = G^T G = L L^T gives
-// A = U^T K U with U = (L^-1 G^T) (x) I3 having orthonormal rows, so the
-// nonzero spectrum of A is that of the 9x9 K = (I (x) L)^T M (I (x) L) and
-// proj(A) = U^T proj(K) U exactly (the 3 translation modes of A are zero).  K
-// has the same block form as A with G_a replaced by the columns of L.
+// the energy does not change under a translation, so A = (Q (x) I) K (Q (x) I)^T
+// with the orthonormal Q of ys_reduced.cuh and a 9x9 K: the nonzero spectrum
+// of A is K's and proj(A) = (Q (x) I) proj(K) (Q (x) I)^T exactly (the 3
+// translation modes of A are zero).
 //
 // Two passes: `snh_eval_kernel` (one thread per tet) computes the gradient and
-// A, runs the PSD test and writes records for the PSD tets; tets that need the
+// K, runs the PSD test and writes records for the PSD tets; tets that need the
 // eigen-solve are compacted into a work list and finished by
 // `snh_project_kernel`, so the expensive path runs without divergence.
 #include "ys_ad.cuh"
 #include "ys_common.cuh"
 #include "ys_eigen.cuh"
+#include "ys_reduced.cuh"
 
 namespace ys {
 
@@ -66,6 +66,22 @@ struct SnhState {
   V3 grad[4];
 };
 
+// Coefficients and energy from F, its cofactors and det = det(Dm).
+__device__ __forceinline__ void snh_material(const ys_snh_args& a, uint32_t t, double det, SnhState& st) {
+  const double mu = a.mu ? a.mu[t] : a.mu_value;
+  const double lam = a.lam ? a.lam[t] : a.lam_value;
+  const double ic = dot(st.f.c[0], st.f.c[0]) + dot(st.f.c[1], st.f.c[1]) + dot(st.f.c[2], st.f.c[2]);
+  const double J = dot(st.f.c[0], st.cof.c[0]);
+  const double alpha = 1.0 + 0.75 * mu / lam;
+  const double vol = det / 6.0;
+  st.s = vol * a.dt * a.dt;
+  st.lam = lam;
+  st.c1 = mu * (1.0 - 1.0 / (ic + 1.0));
+  st.c2 = 2.0 * mu / ((ic + 1.0) * (ic + 1.0));
+  st.c3 = lam * (J - alpha);
+  st.energy = st.s * (0.5 * mu * (ic - 3.0) - 0.5 * mu * log(ic + 1.0) + 0.5 * lam * (J - alpha) * (J - alpha));
+}
+
 __device__ __forceinline__ void snh_state(const ys_snh_args& a, uint32_t t, SnhState& st) {
   const uint4 tv = reinterpret_cast<const uint4*>(a.tets)[t];
   const uint32_t id[4] = {tv.x, tv.y, tv.z, tv.w};
@@ -96,18 +112,7 @@ __device__ __forceinline__ void snh_state(const ys_snh_args& a, uint32_t t, SnhS
   st.cof.c[0] = cross(st.f.c[1], st.f.c[2]);
   st.cof.c[1] = cross(st.f.c[2], st.f.c[0]);
   st.cof.c[2] = cross(st.f.c[0], st.f.c[1]);
-  const double mu = a.mu ? a.mu[t] : a.mu_value;
-  const double lam = a.lam ? a.lam[t] : a.lam_value;
-  const double ic = dot(st.f.c[0], st.f.c[0]) + dot(st.f.c[1], st.f.c[1]) + dot(st.f.c[2], st.f.c[2]);
-  const double J = dot(st.f.c[0], st.cof.c[0]);
-  const double alpha = 1.0 + 0.75 * mu / lam;
-  const double vol = det / 6.0;
-  st.s = vol * a.dt * a.dt;
-  st.lam = lam;
-  st.c1 = mu * (1.0 - 1.0 / (ic + 1.0));
-  st.c2 = 2.0 * mu / ((ic + 1.0) * (ic + 1.0));
-  st.c3 = lam * (J - alpha);
-  st.energy = st.s * (0.5 * mu * (ic - 3.0) - 0.5 * mu * log(ic + 1.0) + 0.5 * lam * (J - alpha) * (J - alpha));
+  snh_material(a, t, det, st);
   // P = c1 F + c3 cof; grad_a = s P G_a^T.
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
@@ -141,79 +146,6 @@ __device__ __forceinline__ void hess_block(const SnhState& st, V3 ga, V3 gb, V3 
     for (int l = 0; l < 3; ++l) blk[k][l] *= st.s;
 }
 
-// Scatter of one instance's projected local Hessian (4 arguments of size 3)
-// into pattern records, merging repeated target arguments and transposing
-// blocks whose row DoF exceeds the column DoF (hessianKernelNoProject.pyx:94-264).
-template <typename BlockFn>
-__device__ __forceinline__ void write_hessian_records(const uint32_t (&code)[4], uint32_t occ0,
-                                                      const uint32_t* __restrict__ record, double* __restrict__ out,
-                                                      BlockFn&& block) {
-  bool dup = false;
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = a + 1; b < 4; ++b) dup |= (code[a] >= 2 && code[a] == code[b]);
-  if (!dup) {
-    // Common case: every target argument is its own group (compile-time indices).
-    uint32_t occ = occ0;
-#pragma unroll
-    for (int ai = 0; ai < 4; ++ai) {
-      if (code[ai] < 2) continue;
-#pragma unroll
-      for (int bi = ai; bi < 4; ++bi) {
-        if (code[bi] < 2) continue;
-        double blk[3][3];
-        block(ai, bi, blk);
-        double* dst = out + record[occ++];
-        const bool upper = code[ai] < code[bi];
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-#pragma unroll
-          for (int l = 0; l < 3; ++l) dst[3 * k + l] = upper ? blk[k][l] : blk[l][k];
-      }
-    }
-    return;
-  }
-  int first[4];
-  int nfirst = 0;
-  int group[4];
-#pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    group[a] = -1;
-    if (code[a] < 2) continue;
-    int gsel = -1;
-    for (int q = 0; q < nfirst; ++q)
-      if (code[first[q]] == code[a]) gsel = q;
-    if (gsel < 0) { first[nfirst] = a; gsel = nfirst++; }
-    group[a] = gsel;
-  }
-  uint32_t occ = occ0;
-  for (int gi = 0; gi < nfirst; ++gi) {
-    for (int gj = gi; gj < nfirst; ++gj) {
-      double acc[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-      for (int a = 0; a < 4; ++a) {
-        if (group[a] != gi) continue;
-        for (int b = 0; b < 4; ++b) {
-          if (group[b] != gj) continue;
-          double blk[3][3];
-          block(a, b, blk);
-#pragma unroll
-          for (int k = 0; k < 3; ++k)
-#pragma unroll
-            for (int l = 0; l < 3; ++l) acc[k][l] += blk[k][l];
-        }
-      }
-      double* dst = out + record[occ];
-      const bool upper = code[first[gi]] < code[first[gj]];
-#pragma unroll
-      for (int k = 0; k < 3; ++k)
-#pragma unroll
-        for (int l = 0; l < 3; ++l) dst[3 * k + l] = upper ? acc[k][l] : acc[l][k];
-      ++occ;
-    }
-  }
-}
-
 __device__ __forceinline__ void write_gradient_records(const uint32_t (&code)[4], uint32_t q0,
                                                        const uint32_t* __restrict__ grec, double* __restrict__ out,
                                                        const V3 (&grad)[4]) {
@@ -233,166 +165,160 @@ __device__ __forceinline__ void load_codes(const ys_term_plan& p, uint32_t t, ui
   for (int a = 0; a < 4; ++a) code[a] = p.codes[(uint64_t)t * p.K + (uint64_t)a * p.slot_stride];
 }
 
-__global__ void __launch_bounds__(128) snh_eval_kernel(const ys_snh_args a) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= a.num_elements) return;
+// The tet in the coordinates of ys_reduced.cuh (QPairs): y_p = sum_a Q[a][p]
+// x_a, Y_p the same of the rest positions.  F = [y0 y1 y2] [Y0 Y1 Y2]^-1, so
+// with R_p the rows of [Y]^-1 the energy's y-gradient is s P R_p and block
+// (p, q) of its 9x9 Hessian K is the block formula with R_p, R_q in place of
+// G_a, G_b.  det(Dm) = -2 det[Y].
+struct SnhReduced {
+  V3 r[3];   // rows R_p
   SnhState st;
-  snh_state(a, t, st);
-  uint32_t code[4];
-  load_codes(a.plan, t, code);
-  if (a.energy) a.energy[t] = st.energy;
-  write_gradient_records(code, a.plan.grad_outer[t], a.plan.grad_record, a.grad_records, st.grad);
-  V3 u[4], v[4];
+};
+
+__device__ __forceinline__ void reduce_pairs(const V3 (&x)[4], V3 (&y)[3]) {
+  const V3 d0 = x[0] - x[1], d1 = x[2] - x[3];
+  y[0] = 0.5 * ((x[0] - x[2]) + (x[1] - x[3]));
+  y[1] = 0.5 * (d0 + d1);
+  y[2] = 0.5 * (d0 - d1);
+}
+
+__device__ __forceinline__ void snh_reduced(const ys_snh_args& a, uint32_t t, SnhReduced& e) {
+  const uint4 tv = reinterpret_cast<const uint4*>(a.tets)[t];
+  const uint32_t id[4] = {tv.x, tv.y, tv.z, tv.w};
+  V3 x[4], rest[4], y[3], w[3];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    u[k] = mul(st.f, st.g[k]);
-    v[k] = mul(st.cof, st.g[k]);
+    x[k] = load3(a.position, id[k]);
+    rest[k] = load3(a.rest, id[k]);
   }
-  auto block = [&](int ai, int bi, double (&blk)[3][3]) {
-    hess_block(st, st.g[ai], st.g[bi], u[ai], u[bi], v[ai], v[bi], blk);
-  };
-  if (a.projection_method >= 1) {
-    double s[78];
+  reduce_pairs(x, y);
+  reduce_pairs(rest, w);
+  const V3 k0 = cross(w[1], w[2]), k1 = cross(w[2], w[0]), k2 = cross(w[0], w[1]);
+  const double det = dot(w[0], k0), inv = 1.0 / det;
+  e.r[0] = inv * k0;
+  e.r[1] = inv * k1;
+  e.r[2] = inv * k2;
+  SnhState& st = e.st;
 #pragma unroll
-    for (int ai = 0; ai < 4; ++ai) {
-#pragma unroll
-      for (int bi = 0; bi <= ai; ++bi) {
-        double blk[3][3];
-        hess_block(st, st.g[ai], st.g[bi], u[ai], u[bi], v[ai], v[bi], blk);
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-#pragma unroll
-          for (int l = 0; l < 3; ++l) {
-            const int r = 3 * ai + k, c = 3 * bi + l;
-            if (c <= r) s[tri(r, c)] = blk[k][l];
-          }
-      }
-    }
-    if (!psd_test_packed<12>(s)) {
-      const uint32_t slot = atomicAdd(a.work_count, 1u);
-      a.work_list[slot] = t;
-      return;
-    }
-  }
-  write_hessian_records(code, a.plan.coord_outer[t], a.plan.record, a.block_records, block);
+  for (int j = 0; j < 3; ++j) st.f.c[j] = comp(e.r[0], j) * y[0] + comp(e.r[1], j) * y[1] + comp(e.r[2], j) * y[2];
+  st.cof.c[0] = cross(st.f.c[1], st.f.c[2]);
+  st.cof.c[1] = cross(st.f.c[2], st.f.c[0]);
+  st.cof.c[2] = cross(st.f.c[0], st.f.c[1]);
+  snh_material(a, t, -2.0 * det, st);
 }
 
-// Lower Cholesky of a 3x3 SPD matrix W given by its entries.
-__device__ __forceinline__ bool chol3(double w00, double w01, double w02, double w11, double w12, double w22,
-                                      double (&l)[3][3]) {
-  if (!(w00 > 0.0)) return false;
-  const double l00 = sqrt(w00);
-  const double l10 = w01 / l00, l20 = w02 / l00;
-  const double d1 = w11 - l10 * l10;
-  if (!(d1 > 0.0)) return false;
-  const double l11 = sqrt(d1);
-  const double l21 = (w12 - l20 * l10) / l11;
-  const double d2 = w22 - l20 * l20 - l21 * l21;
-  if (!(d2 > 0.0)) return false;
-  const double l22 = sqrt(d2);
-  l[0][0] = l00; l[0][1] = 0.0; l[0][2] = 0.0;
-  l[1][0] = l10; l[1][1] = l11; l[1][2] = 0.0;
-  l[2][0] = l20; l[2][1] = l21; l[2][2] = l22;
-  return true;
-}
-
-__device__ __forceinline__ void snh_project_one(const ys_snh_args& a, uint32_t t, double* __restrict__ stash,
-                                                int stride) {
-  SnhState st;
-  snh_state(a, t, st);
-  uint32_t code[4];
-  load_codes(a.plan, t, code);
-  // W = G^T G (3x3 over the column index j).
-  double w[3][3];
-#pragma unroll
-  for (int j = 0; j < 3; ++j)
-#pragma unroll
-    for (int m = 0; m < 3; ++m) {
-      double acc = 0.0;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) acc += comp(st.g[k], j) * comp(st.g[k], m);
-      w[j][m] = acc;
-    }
-  double l[3][3];
-  const bool ok = chol3(w[0][0], w[0][1], w[0][2], w[1][1], w[1][2], w[2][2], l);
-  if (!ok) {
-    // Degenerate rest tetrahedron: no finite projection exists; keep A as is.
-    V3 u[4], v[4];
-    for (int k = 0; k < 4; ++k) { u[k] = mul(st.f, st.g[k]); v[k] = mul(st.cof, st.g[k]); }
-    auto raw = [&](int ai, int bi, double (&blk)[3][3]) {
-      hess_block(st, st.g[ai], st.g[bi], u[ai], u[bi], v[ai], v[bi], blk);
-    };
-    write_hessian_records(code, a.plan.coord_outer[t], a.plan.record, a.block_records, raw);
-    return;
-  }
-  // Columns of L play the role of G in K.
-  V3 lc[3], lu[3], lv[3];
+// K (packed upper 9x9).
+__device__ __forceinline__ void snh_reduced_hessian(const SnhReduced& e, double (&k)[45]) {
+  V3 u[3], v[3];
 #pragma unroll
   for (int p = 0; p < 3; ++p) {
-    lc[p] = {l[0][p], l[1][p], l[2][p]};
-    lu[p] = mul(st.f, lc[p]);
-    lv[p] = mul(st.cof, lc[p]);
+    u[p] = mul(e.st.f, e.r[p]);
+    v[p] = mul(e.st.cof, e.r[p]);
   }
-  // Q = G L^-T: Q[a][p] = sum_j G[a][j] (L^-1)[p][j]; solve L y = G_a per vertex.
-  constexpr int QS = project_stash_doubles<9>();
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const double g0 = st.g[k].x, g1 = st.g[k].y, g2 = st.g[k].z;
-    const double y0 = g0 / l[0][0];
-    const double y1 = (g1 - l[1][0] * y0) / l[1][1];
-    const double y2 = (g2 - l[2][0] * y0 - l[2][1] * y1) / l[2][2];
-    stash[(QS + 3 * k) * stride] = y0;
-    stash[(QS + 3 * k + 1) * stride] = y1;
-    stash[(QS + 3 * k + 2) * stride] = y2;
-  }
-  // K (9x9, packed upper triangle in registers), projected in place.
-  double kmat[45];
 #pragma unroll
   for (int p = 0; p < 3; ++p)
 #pragma unroll
     for (int q = p; q < 3; ++q) {
       double blk[3][3];
-      hess_block(st, lc[p], lc[q], lu[p], lu[q], lv[p], lv[q], blk);
+      hess_block(e.st, e.r[p], e.r[q], u[p], u[q], v[p], v[q], blk);
 #pragma unroll
-      for (int k = 0; k < 3; ++k)
+      for (int r = 0; r < 3; ++r)
 #pragma unroll
-        for (int m = 0; m < 3; ++m)
-          if (3 * p + k <= 3 * q + m) kmat[utri<9>(3 * p + k, 3 * q + m)] = blk[k][m];
+        for (int c = 0; c < 3; ++c)
+          if (3 * p + r <= 3 * q + c) k[utri<9>(3 * p + r, 3 * q + c)] = blk[r][c];
     }
-  project_negative_modes<9>(kmat, a.projection_method, stash, stride);
-  double qm[4][3];
+}
+
+constexpr int kEvalThreads = 128;
+
+// The reference's PSD test of the 12x12 Hessian of the stashed K.
+__device__ __noinline__ int snh_psd_full(const double* stash) {
+  double s[78];
+  vertex_lower<QPairs, 4, 4>(stash, kEvalThreads, s);
+  return psd_test_packed<12>(s) ? 1 : 0;
+}
+
+__global__ void __launch_bounds__(kEvalThreads, 4) snh_eval_kernel(const ys_snh_args a) {
+  const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool live = i0 < a.num_elements;
+  const uint32_t t = live ? i0 : a.num_elements - 1;  // whole warps: the records are written by all lanes
+  uint32_t code[4];
+  load_codes(a.plan, t, code);
+  SnhReduced e;
+  snh_reduced(a, t, e);
+  if (live && a.energy) a.energy[t] = e.st.energy;
+  if (live) {
+    V3 gy[3], grad[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k)
+    for (int p = 0; p < 3; ++p) gy[p] = e.st.s * (e.st.c1 * mul(e.st.f, e.r[p]) + e.st.c3 * mul(e.st.cof, e.r[p]));
 #pragma unroll
-    for (int p = 0; p < 3; ++p) qm[k][p] = stash[(QS + 3 * k + p) * stride];
-  auto block = [&](int ai, int bi, double (&blk)[3][3]) {
+    for (int k = 0; k < 4; ++k)
+      grad[k] = QPairs::q(k, 0) * gy[0] + QPairs::q(k, 1) * gy[1] + QPairs::q(k, 2) * gy[2];
+    write_gradient_records(code, a.plan.grad_outer[t], a.plan.grad_record, a.grad_records, grad);
+  }
+  // K waits in shared memory (thread-interleaved) while the PSD test runs in
+  // registers: 45 + 45 doubles live at once would halve the resident warps.
+  extern __shared__ double eval_stash[];
+  double* stash = eval_stash + threadIdx.x;
+  double scale = 0.0;
+  {
+    double k[45];
+    snh_reduced_hessian(e, k);
+    scale = vertex_scale<QPairs, 4>(k);
 #pragma unroll
-    for (int k = 0; k < 3; ++k)
-#pragma unroll
-      for (int m = 0; m < 3; ++m) {
-        double acc = 0.0;
-#pragma unroll
-        for (int p = 0; p < 3; ++p)
-#pragma unroll
-          for (int q = 0; q < 3; ++q) acc += qm[ai][p] * qm[bi][q] * kmat[utri<9>(3 * p + k, 3 * q + m)];
-        blk[k][m] = acc;
-      }
-  };
-  write_hessian_records(code, a.plan.coord_outer[t], a.plan.record, a.block_records, block);
+    for (int i = 0; i < 45; ++i) stash[i * kEvalThreads] = k[i];
+  }
+  bool write = live;
+  if (a.projection_method >= 1) {
+    asm volatile("" ::: "memory");
+    double s[45];
+    vertex_lower<QPairs, 4, 3>(stash, kEvalThreads, s);
+    int psd = psd_test_leading<9>(s, scale);
+    if (psd < 0) psd = snh_psd_full(stash);
+    if (live && !psd) {
+      const uint32_t slot = atomicAdd(a.work_count, 1u);
+      a.work_list[slot] = t;
+      write = false;
+    }
+  }
+  asm volatile("" ::: "memory");
+  VertexRows<QPairs, 4> rows{stash, kEvalThreads};
+  write_block_records<4, true>(write, code, a.plan.coord_outer[t], a.plan.record, a.block_records,
+                         eval_stash + 45 * kEvalThreads, rows);
 }
 
 constexpr int kProjThreads = 64;
 
-// Per-thread shared-memory stash of the projection (original K, reflectors,
-// Q), thread-interleaved.
-constexpr int kProjStash = project_stash_doubles<9>() + 12;
+// Per-thread shared-memory stash of the projection (original K and
+// reflectors), thread-interleaved.
+constexpr int kProjStash = project_stash_doubles<9>();
 
 __global__ void __launch_bounds__(kProjThreads) snh_project_kernel(const ys_snh_args a) {
   extern __shared__ double proj_stash[];
   double* stash = proj_stash + threadIdx.x;
   const uint32_t count = *a.work_count;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
-    snh_project_one(a, a.work_list[i], stash, blockDim.x);
+  // whole warps (lanes past the list repeat its last element and write nothing)
+  for (uint32_t base = blockIdx.x * kProjThreads + (threadIdx.x & ~31u); base < count;
+       base += gridDim.x * kProjThreads) {
+    const uint32_t i = base + (threadIdx.x & 31u);
+    const bool live = i < count;
+    const uint32_t t = a.work_list[live ? i : count - 1];
+    {
+      double k[45];
+      {
+        SnhReduced e;
+        snh_reduced(a, t, e);
+        snh_reduced_hessian(e, k);
+      }
+#pragma unroll
+      for (int j = 0; j < 45; ++j) stash[j * blockDim.x] = k[j];
+      project_negative_modes<9, true>(k, a.projection_method, stash, blockDim.x);
+    }
+    uint32_t code[4];
+    load_codes(a.plan, t, code);
+    VertexRows<QPairs, 4> rows{stash, (int)blockDim.x};
+    write_block_records<4, false>(live, code, a.plan.coord_outer[t], a.plan.record, a.block_records, nullptr, rows);
+  }
 }
 
 // Unprojected 12x12 local Hessian A of every tet (packed upper, 78 doubles),
@@ -764,8 +690,10 @@ int32_t ys_snh_eval(const ys_snh_args* args, void* stream) {
     YS_REQUIRE(a.work_list && a.work_count, YS_ERR_INVALID, "projection needs work_list/work_count");
     YS_CUDA_TRY(cudaMemsetAsync(a.work_count, 0, sizeof(uint32_t), s));
   }
-  const unsigned grid = ys::grid_for(a.num_elements, 128);
-  ys::snh_eval_kernel<<<grid, 128, 0, s>>>(a);
+  const unsigned grid = ys::grid_for(a.num_elements, ys::kEvalThreads);
+  const size_t esmem = sizeof(double) * (45 + ys::kRecordRow) * ys::kEvalThreads;
+  YS_CUDA_TRY(cudaFuncSetAttribute(ys::snh_eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)esmem));
+  ys::snh_eval_kernel<<<grid, ys::kEvalThreads, esmem, s>>>(a);
   YS_CHECK_LAUNCH();
   if (a.projection_method >= 1) {
     // The work count stays on the device: a grid-stride launch sized to the

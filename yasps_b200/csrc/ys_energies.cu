@@ -16,10 +16,15 @@
 // second-order forward-mode differentiation (ys_ad.cuh); the local Hessian
 // is projected like the SNH one (LDL^T PSD test, then the negative modes) and
 // scattered with the NoProject merge rules into pattern records.
+//
+// ys_energy_eval evaluates the closed-form Hessians of the reduce() members in
+// translation-free coordinates (ys_reduced.cuh); the HD<N> formulas serve the
+// energy totals, the coupled (affine-body) pairs and the Jacobians.
 #include <type_traits>
 
 #include "ys_ad.cuh"
 #include "ys_common.cuh"
+#include "ys_reduced.cuh"
 
 namespace ys {
 
@@ -49,8 +54,20 @@ __device__ __forceinline__ HD<N> barrier_of(const HD<N>& d, double dhat, double 
   return hd_apply(d, f, df, d2f);
 }
 
+template <int A>
+__device__ __forceinline__ D3v pt(const Pts<A>& x, int a) {
+  return d3v(x.p[a]);
+}
+
+// kAlwaysProjects: nearly every element (an active barrier) is indefinite.
 struct PointPoint {
   static constexpr int A = 2;
+  static constexpr bool kAlwaysProjects = true;
+  using Q = QTwo;
+  __device__ __forceinline__ static void reduce(const ys_energy_args& a, uint32_t, const Pts<A>& x, const Pts<A>&,
+                                                Reduced<A>& e) {
+    point_barrier(kSqrt1_2 * (pt(x, 0) - pt(x, 1)), a.values[0], a.values[1], e);
+  }
   template <int N>
   __device__ static HD<N> eval(const ys_energy_args& a, uint32_t, const Pts<A>& x, const Pts<A>&) {
     const HV<N> p0 = hv_var<N>(x.p[0], 0), p1 = hv_var<N>(x.p[1], 3);
@@ -61,6 +78,14 @@ struct PointPoint {
 
 struct PointEdge {
   static constexpr int A = 3;
+  static constexpr bool kAlwaysProjects = true;
+  using Q = QThree;
+  __device__ __forceinline__ static void reduce(const ys_energy_args& a, uint32_t, const Pts<A>& x, const Pts<A>&,
+                                                Reduced<A>& e) {
+    const D3v y[2] = {kSqrt1_6 * ((pt(x, 0) - pt(x, 1)) + (pt(x, 0) - pt(x, 2))),
+                      kSqrt1_2 * (pt(x, 1) - pt(x, 2))};
+    line_barrier(y, a.values[0], a.values[1], e);
+  }
   template <int N>
   __device__ static HD<N> eval(const ys_energy_args& a, uint32_t, const Pts<A>& x, const Pts<A>&) {
     const HV<N> p0 = hv_var<N>(x.p[0], 0), p1 = hv_var<N>(x.p[1], 3), p2 = hv_var<N>(x.p[2], 6);
@@ -72,6 +97,15 @@ struct PointEdge {
 
 struct PointTriangle {
   static constexpr int A = 4;
+  static constexpr bool kAlwaysProjects = true;
+  using Q = QPointTriangle;
+  __device__ __forceinline__ static void reduce(const ys_energy_args& a, uint32_t, const Pts<A>& x, const Pts<A>&,
+                                                Reduced<A>& e) {
+    const D3v y[3] = {kSqrt1_12 * ((pt(x, 0) - pt(x, 1)) + (pt(x, 0) - pt(x, 2)) + (pt(x, 0) - pt(x, 3))),
+                      kSqrt1_2 * (pt(x, 1) - pt(x, 2)),
+                      kSqrt1_6 * ((pt(x, 1) - pt(x, 3)) + (pt(x, 2) - pt(x, 3)))};
+    plane_barrier(y, 4.0 / 3.0, a.values[0], a.values[1], e);
+  }
   template <int N>
   __device__ static HD<N> eval(const ys_energy_args& a, uint32_t, const Pts<A>& x, const Pts<A>&) {
     const HV<N> p0 = hv_var<N>(x.p[0], 0), p1 = hv_var<N>(x.p[1], 3), p2 = hv_var<N>(x.p[2], 6),
@@ -84,6 +118,14 @@ struct PointTriangle {
 
 struct EdgeEdge {
   static constexpr int A = 4;
+  static constexpr bool kAlwaysProjects = true;
+  using Q = QPairs;
+  __device__ __forceinline__ static void reduce(const ys_energy_args& a, uint32_t, const Pts<A>& x, const Pts<A>&,
+                                                Reduced<A>& e) {
+    const D3v d0 = pt(x, 0) - pt(x, 1), d1 = pt(x, 2) - pt(x, 3);
+    const D3v y[3] = {0.5 * ((pt(x, 0) - pt(x, 2)) + (pt(x, 1) - pt(x, 3))), 0.5 * (d0 + d1), 0.5 * (d0 - d1)};
+    plane_barrier(y, 1.0, a.values[0], a.values[1], e);
+  }
   template <int N>
   __device__ static HD<N> eval(const ys_energy_args& a, uint32_t, const Pts<A>& x, const Pts<A>&) {
     const HV<N> p0 = hv_var<N>(x.p[0], 0), p1 = hv_var<N>(x.p[1], 3), p2 = hv_var<N>(x.p[2], 6),
@@ -116,6 +158,18 @@ __device__ __forceinline__ double dihedral(const double (&q0)[3], const double (
 
 struct Bending {
   static constexpr int A = 4;
+  static constexpr bool kAlwaysProjects = false;
+  using Q = QHinge;
+  __device__ __forceinline__ static void reduce(const ys_energy_args& a, uint32_t, const Pts<A>& x, const Pts<A>& r,
+                                                Reduced<A>& e) {
+    const double theta = dihedral(x.p[0], x.p[1], x.p[2], x.p[3]);
+    const double theta0 = dihedral(r.p[0], r.p[1], r.p[2], r.p[3]);
+    const D3v l = pt(r, 1) - pt(r, 0);
+    const double dt = a.values[1];
+    const D3v y[3] = {0.5 * ((pt(x, 2) - pt(x, 0)) + (pt(x, 3) - pt(x, 1))), kSqrt1_2 * (pt(x, 1) - pt(x, 0)),
+                      kSqrt1_2 * (pt(x, 3) - pt(x, 2))};
+    hinge_energy(y, a.values[0] * sqrt(dot(l, l)) * dt * dt, theta - theta0, e);
+  }
   template <int N>
   __device__ static HD<N> eval(const ys_energy_args& a, uint32_t, const Pts<A>& x, const Pts<A>& r) {
     const HV<N> q0 = hv_var<N>(x.p[0], 0), q1 = hv_var<N>(x.p[1], 3), q2 = hv_var<N>(x.p[2], 6),
@@ -184,8 +238,38 @@ __device__ __forceinline__ void membrane_f(const Pts<3>& x, const double (&minv)
   f1 = minv[0][1] * x10 + minv[1][1] * x20;
 }
 
+// Columns f0, f1 of F and their coordinates m over y (QThree): x1 - x0 =
+// -sqrt(3/2) y0 + y1 / sqrt2, x2 - x0 = -sqrt(3/2) y0 - y1 / sqrt2.
+__device__ __forceinline__ void membrane_reduced(const Pts<3>& x, const double (&minv)[2][2], D3v (&f)[2],
+                                                 double (&m)[2][2]) {
+  const D3v x10 = pt(x, 1) - pt(x, 0), x20 = pt(x, 2) - pt(x, 0);
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    f[j] = minv[0][j] * x10 + minv[1][j] * x20;
+    m[0][j] = -kSqrt3_2 * (minv[0][j] + minv[1][j]);
+    m[1][j] = kSqrt1_2 * (minv[0][j] - minv[1][j]);
+  }
+}
+
 struct BaraffWitkin {
   static constexpr int A = 3;
+  static constexpr bool kAlwaysProjects = false;
+  using Q = QThree;
+  __device__ __forceinline__ static void reduce(const ys_energy_args& a, uint32_t, const Pts<A>& x, const Pts<A>& r,
+                                                Reduced<A>& e) {
+    double minv[2][2], area, m[2][2];
+    rest_frame(r, minv, area);
+    D3v f[2];
+    membrane_reduced(x, minv, f, m);
+    const double cc = dot(f[0], f[1]), au = dot(f[0], f[0]), av = dot(f[1], f[1]);
+    const double iu = sqrt(au), iv = sqrt(av);
+    const double uc = iu < 1.0 ? 0.01 : 1.0, vc = iv < 1.0 ? 0.01 : 1.0;
+    const double dt = a.values[3], w = a.values[2] * area * dt * dt;
+    const double ws = w * a.values[0], wc = w * a.values[1];
+    e.v = ws * (uc * (iu - 1.0) * (iu - 1.0) + vc * (iv - 1.0) * (iv - 1.0)) + wc * cc * cc;
+    metric_energy(f[0], f[1], m, ws * uc * (iu - 1.0) / iu, ws * vc * (iv - 1.0) / iv, 2.0 * wc * cc,
+                  0.5 * ws * uc / (iu * au), 0.5 * ws * vc / (iv * av), 0.0, 2.0 * wc, e);
+  }
   template <int N>
   __device__ static HD<N> eval(const ys_energy_args& a, uint32_t, const Pts<A>& x, const Pts<A>& r) {
     double minv[2][2], area;
@@ -205,6 +289,21 @@ struct BaraffWitkin {
 // psi = mu tr(E^2) + lam/2 tr(E)^2, E = (F^T F - I) / 2, on the same rest frame.
 struct StvkMembrane {
   static constexpr int A = 3;
+  static constexpr bool kAlwaysProjects = false;
+  using Q = QThree;
+  __device__ __forceinline__ static void reduce(const ys_energy_args& a, uint32_t, const Pts<A>& x, const Pts<A>& r,
+                                                Reduced<A>& e) {
+    double minv[2][2], area, m[2][2];
+    rest_frame(r, minv, area);
+    D3v f[2];
+    membrane_reduced(x, minv, f, m);
+    const double e00 = 0.5 * (dot(f[0], f[0]) - 1.0), e11 = 0.5 * (dot(f[1], f[1]) - 1.0), e01 = 0.5 * dot(f[0], f[1]);
+    const double tr = e00 + e11, dt = a.values[3], w = a.values[2] * area * dt * dt;
+    const double wm = w * a.values[0], wl = w * a.values[1];
+    e.v = wm * (e00 * e00 + e11 * e11 + 2.0 * e01 * e01) + 0.5 * wl * tr * tr;
+    metric_energy(f[0], f[1], m, wm * e00 + 0.5 * wl * tr, wm * e11 + 0.5 * wl * tr, 2.0 * wm * e01,
+                  0.5 * wm + 0.25 * wl, 0.5 * wm + 0.25 * wl, 0.25 * wl, wm, e);
+  }
   template <int N>
   __device__ static HD<N> eval(const ys_energy_args& a, uint32_t, const Pts<A>& x, const Pts<A>& r) {
     double minv[2][2], area;
@@ -379,9 +478,52 @@ __device__ __forceinline__ void step_inputs(const Pts<A>& x, const Pts<A>& r, HV
   }
 }
 
+// The same energy in closed form: rel = sum_k c_k (x_k - x_old,k) is linear,
+// so the gradient of vertex k is c_k g and the Hessian block (k, l) is
+// c_k c_l h with the 3x3 h = d2E/drel2 (packed upper).
+struct FrictionLocal {
+  double v;
+  double g[3];
+  double h[6];
+};
+__device__ __forceinline__ FrictionLocal friction_local(const ys_energy_args& a, const double* q, const D3v& rel) {
+  const D3v t0 = {q[2], q[3], q[4]}, t1 = {q[5], q[6], q[7]};
+  const double u0 = dot(t0, rel), u1 = dot(t1, rel), y2 = u0 * u0 + u1 * u1;
+  const double fdhat = a.values[0], dt = a.values[1], w = a.values[2] * q[8];
+  const double eps = sqrt(fdhat) * dt, fric_dhat = fdhat * dt * dt;
+  const double y = sqrt(y2 + 1e-16), iy = 1.0 / y;
+  double phi, p1, p2;  // phi(y2) and its derivatives in y2
+  if (y2 > fric_dhat) {
+    phi = y;
+    p1 = 0.5 * iy;
+    p2 = -0.25 * iy * iy * iy;
+  } else {
+    const double ie = 1.0 / (3.0 * eps * eps);
+    phi = (y2 / eps + eps / 3.0) - ie * (y2 * y);
+    p1 = 1.0 / eps - ie * (y + 0.5 * y2 * iy);
+    p2 = -ie * (iy - 0.25 * y2 * iy * iy * iy);
+  }
+  FrictionLocal f;
+  f.v = w * phi;
+  const D3v v = u0 * t0 + u1 * t1;
+  const double c1 = 2.0 * w * p1, c2 = 4.0 * w * p2;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    f.g[i] = c1 * at(v, i);
+#pragma unroll
+    for (int j = i; j < 3; ++j)
+      f.h[utri<3>(i, j)] = c1 * (at(t0, i) * at(t0, j) + at(t1, i) * at(t1, j)) + c2 * at(v, i) * at(v, j);
+  }
+  return f;
+}
+
 // Point-triangle (:73-182): lagged (beta1, beta2) of the closest point.
 struct FrictionPT {
   static constexpr int A = 4;
+  static constexpr bool kFriction = true;
+  __device__ __forceinline__ static void weights(const double* q, double (&c)[A]) {
+    c[0] = 1.0; c[1] = q[0] + q[1] - 1.0; c[2] = -q[0]; c[3] = -q[1];
+  }
   template <int N>
   __device__ static HD<N> eval(const ys_energy_args& a, uint32_t t, const Pts<A>& x, const Pts<A>& r) {
     const double* q = a.params + (uint64_t)t * a.param_stride;
@@ -394,6 +536,10 @@ struct FrictionPT {
 // Point-edge (:188-276): lagged eta of the closest point on the edge.
 struct FrictionPE {
   static constexpr int A = 3;
+  static constexpr bool kFriction = true;
+  __device__ __forceinline__ static void weights(const double* q, double (&c)[A]) {
+    c[0] = 1.0; c[1] = q[0] - 1.0; c[2] = -q[0];
+  }
   template <int N>
   __device__ static HD<N> eval(const ys_energy_args& a, uint32_t t, const Pts<A>& x, const Pts<A>& r) {
     const double* q = a.params + (uint64_t)t * a.param_stride;
@@ -406,6 +552,10 @@ struct FrictionPE {
 // Edge-edge (:283-405): lagged (gamma1, gamma2) of the closest points.
 struct FrictionEE {
   static constexpr int A = 4;
+  static constexpr bool kFriction = true;
+  __device__ __forceinline__ static void weights(const double* q, double (&c)[A]) {
+    c[0] = 1.0 - q[0]; c[1] = q[0]; c[2] = q[1] - 1.0; c[3] = -q[1];
+  }
   template <int N>
   __device__ static HD<N> eval(const ys_energy_args& a, uint32_t t, const Pts<A>& x, const Pts<A>& r) {
     const double* q = a.params + (uint64_t)t * a.param_stride;
@@ -418,6 +568,10 @@ struct FrictionEE {
 // Point-point (:411-500).
 struct FrictionPP {
   static constexpr int A = 2;
+  static constexpr bool kFriction = true;
+  __device__ __forceinline__ static void weights(const double* q, double (&c)[A]) {
+    c[0] = 1.0; c[1] = -1.0;
+  }
   template <int N>
   __device__ static HD<N> eval(const ys_energy_args& a, uint32_t t, const Pts<A>& x, const Pts<A>& r) {
     const double* q = a.params + (uint64_t)t * a.param_stride;
@@ -514,12 +668,86 @@ __device__ __forceinline__ void finish_element(const Args& a, uint32_t t, const 
   write_records<A>(code, a.plan.coord_outer[t], a.plan.record, a.block_records, h);
 }
 
+template <class E, class = void>
+struct IsFriction : std::false_type {};
+template <class E>
+struct IsFriction<E, std::void_t<decltype(E::kFriction)>> : std::bool_constant<E::kFriction> {};
+
+// Size of the eigenvalue problem of an energy's projection.
+template <class E>
+constexpr int energy_modes() {
+  return IsFriction<E>::value ? 3 : 3 * (E::A - 1);
+}
+
+__device__ __forceinline__ void store3(double* dst, double x, double y, double z) {
+  dst[0] = x;
+  dst[1] = y;
+  dst[2] = z;
+}
+
+// Projection of a friction element, whose 3A x 3A Hessian is (c c^T) (x) h:
+// its nonzero eigenvalues are |c|^2 times h's, so h's negative modes are
+// projected.  The PSD test runs on the 3A x 3A matrix, as the reference's:
+// its tolerance is absolute for small entries, so a test of h would decide
+// differently near it.
+template <int A>
+__device__ __forceinline__ void friction_project(FrictionLocal& f, const double (&c)[A], int method, double* stash) {
+  if (method < 1) return;
+  constexpr int N = 3 * A;
+  double s[N * (N + 1) / 2];
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+#pragma unroll
+    for (int j = 0; j <= i; ++j) s[tri(i, j)] = (c[i / 3] * c[j / 3]) * f.h[sym<3>(i % 3, j % 3)];
+  if (!psd_test_packed<N>(s)) project_negative_modes<3>(f.h, method, stash, blockDim.x);
+}
+
+// Projection of an element in reduced coordinates (ys_reduced.cuh); K is left
+// in the shared stash.  It waits there while the PSD test of the vertex-space
+// matrix holds its 78 entries in registers.
+template <class Q, int A>
+__device__ __forceinline__ void reduced_project(Reduced<A>& e, int method, double* stash) {
+  constexpr int N = Reduced<A>::N, H = Reduced<A>::H;
+  const int stride = blockDim.x;
+#pragma unroll
+  for (int i = 0; i < H; ++i) stash[i * stride] = e.k[i];
+  if (method < 1) return;
+  asm volatile("" ::: "memory");  // the test reads K back: its registers are free
+  double s[3 * A * (3 * A + 1) / 2];
+  vertex_lower<Q, A, A>(stash, stride, s);
+  if (psd_test_packed<3 * A>(s)) return;
+  asm volatile("" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < H; ++i) e.k[i] = stash[i * stride];
+  project_negative_modes<N, true>(e.k, method, stash, stride);
+}
+
+// Blocks c_a c_b h of a friction element.
+template <int A>
+struct FrictionRows {
+  const double (&c)[A];
+  const double (&h)[6];
+  __device__ __forceinline__ void row(int) {}
+  __device__ __forceinline__ void block(int a, int b, double (&blk)[3][3]) const {
+    const double w = c[a] * c[b];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+      for (int l = 0; l < 3; ++l) blk[k][l] = w * h[sym<3>(k, l)];
+  }
+};
+
+// A thread an element.  The closed-form Hessian over A - 1 vectors
+// (ys_reduced.cuh) replaces second-order differentiation numbers over 3A
+// inputs, which spilled 2-10 KB a thread.
 template <class E>
 __global__ void __launch_bounds__(kEnergyThreads) energy_kernel(const ys_energy_args a) {
-  constexpr int A = E::A, N = 3 * A;
+  constexpr int A = E::A;
   extern __shared__ double energy_stash[];
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= a.num_elements) return;
+  double* const rows = energy_stash + project_stash_doubles<energy_modes<E>()>() * kEnergyThreads;
+  const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool live = i0 < a.num_elements;
+  const uint32_t t = live ? i0 : a.num_elements - 1;  // whole warps: the records are written by all lanes
   Pts<A> x, r;
 #pragma unroll
   for (int k = 0; k < A; ++k) {
@@ -528,8 +756,46 @@ __global__ void __launch_bounds__(kEnergyThreads) energy_kernel(const ys_energy_
     if (a.rest.num_children) load_point(a.rest, id, r.p[k]);
     else r.p[k][0] = r.p[k][1] = r.p[k][2] = 0.0;
   }
-  const HD<N> e = E::template eval<N>(a, t, x, r);
-  finish_element<A>(a, t, e, energy_stash + threadIdx.x);
+  uint32_t code[A];
+  load_arg_codes<A>(a.plan, t, code);
+  uint32_t gq = a.plan.grad_outer[t];
+  const uint32_t occ0 = a.plan.coord_outer[t];
+  if constexpr (IsFriction<E>::value) {
+    const double* q = a.params + (uint64_t)t * a.param_stride;
+    double c[A];
+    E::weights(q, c);
+    D3v rel = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < A; ++k) rel = rel + c[k] * (pt(x, k) - pt(r, k));
+    FrictionLocal f = friction_local(a, q, rel);
+    if (live && a.energy) a.energy[t] = f.v;
+#pragma unroll
+    for (int k = 0; k < A; ++k)
+      if (live && code[k] >= 2) store3(a.grad_records + a.plan.grad_record[gq++], c[k] * f.g[0], c[k] * f.g[1], c[k] * f.g[2]);
+    friction_project<A>(f, c, a.projection_method, energy_stash + threadIdx.x);
+    write_block_records<A, true>(live, code, occ0, a.plan.record, a.block_records, rows, FrictionRows<A>{c, f.h});
+  } else {
+    using Q = typename E::Q;
+    constexpr int M = A - 1, N = 3 * M;
+    Reduced<A> e;
+    E::reduce(a, t, x, r, e);
+    if (live && a.energy) a.energy[t] = e.v;
+#pragma unroll
+    for (int k = 0; k < A; ++k) {
+      if (!live || code[k] < 2) continue;
+      double g[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+      for (int p = 0; p < M; ++p)
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+          if (Q::q(k, p) != 0.0) g[c] += Q::q(k, p) * e.g[3 * p + c];
+      store3(a.grad_records + a.plan.grad_record[gq++], g[0], g[1], g[2]);
+    }
+    reduced_project<Q, A>(e, a.projection_method, energy_stash + threadIdx.x);
+    asm volatile("" ::: "memory");
+    VertexRows<Q, A> v{energy_stash + threadIdx.x, (int)blockDim.x};
+    write_block_records<A, !E::kAlwaysProjects>(live, code, occ0, a.plan.record, a.block_records, rows, v);
+  }
 }
 
 // Per-element energy only (line search): the same formulas on HD<0> numbers.
@@ -591,8 +857,8 @@ static int32_t launch_energy_value(const ys_energy_args& a, cudaStream_t s) {
 template <class E>
 static int32_t launch_energy(const ys_energy_args& a, cudaStream_t s) {
   YS_REQUIRE(a.arity == (uint32_t)E::A, YS_ERR_INVALID, "arity does not match the energy kind");
-  constexpr int N = 3 * E::A;
-  const size_t smem = sizeof(double) * project_stash_doubles<N>() * kEnergyThreads;
+  const size_t smem =
+      sizeof(double) * (project_stash_doubles<energy_modes<E>()>() + kRecordRow) * kEnergyThreads;
   YS_CUDA_TRY(cudaFuncSetAttribute(energy_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   energy_kernel<E><<<grid_for(a.num_elements, kEnergyThreads), kEnergyThreads, smem, s>>>(a);
   YS_CHECK_LAUNCH();
