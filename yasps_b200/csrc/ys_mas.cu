@@ -97,13 +97,14 @@ __device__ __forceinline__ void static_for(F&& f) {
 
 // Dense assembly + in-place Gauss-Jordan inverse of one domain per CTA.
 // T: register tile edge (domain size <= 16 T).
-// PB pivots per blocked step (2: fits 128 registers, two CTAs per SM for the
-// 96-DoF domains; 4: the 128-DoF tile, one CTA per SM).
+// PB pivots per blocked step.  T <= 6 (the 96-DoF domains) runs the symmetric
+// form below and fits two CTAs an SM.
 template <int T, int PB>
-__global__ void __launch_bounds__(kInvThreads, PB == 2 ? 2 : 1) mas_domain_inverse(MasDev M) {
+__global__ void __launch_bounds__(kInvThreads, T <= 6 ? 2 : 1) mas_domain_inverse(MasDev M) {
   extern __shared__ double A[];  // n*n
   __shared__ double colb[2][128 * 4];
   __shared__ double rowb[2][4 * 128];
+  __shared__ double wbuf[T <= 6 ? 128 * 4 : 1];
   __shared__ double dinv[128];
   __shared__ int bad;
   const uint32_t d = blockIdx.x;
@@ -112,13 +113,33 @@ __global__ void __launch_bounds__(kInvThreads, PB == 2 ? 2 : 1) mas_domain_inver
   if (threadIdx.x == 0) bad = 0;
   __syncthreads();
   const uint32_t e0 = M.dom_entry_ptr[d], e1 = M.dom_entry_ptr[d + 1];
-  for (uint64_t t = (uint64_t)e0 * 9 + threadIdx.x; t < (uint64_t)e1 * 9; t += blockDim.x) {
-    const uint64_t e = t / 9;
-    const int el = (int)(t % 9), k = el / 3, m = el % 3;
-    const uint32_t li = M.dom_entry[3 * e], lj = M.dom_entry[3 * e + 1], bi = M.dom_entry[3 * e + 2];
-    const double v = level_block(M, bi)[el];
-    A[(3 * li + k) * n + 3 * lj + m] = v;
-    if (li != lj) A[(3 * lj + m) * n + 3 * li + k] = v;
+  // four entries a thread in flight: an entry is two dependent loads, and one
+  // at a time they took a quarter of the kernel
+  constexpr int kAhead = 4;
+  const uint32_t values = 9 * (e1 - e0);
+  for (uint32_t t0 = threadIdx.x; t0 < values; t0 += kAhead * kInvThreads) {
+    uint32_t li[kAhead], lj[kAhead], bi[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const uint32_t t = t0 + u * kInvThreads, e = e0 + (t < values ? t : t0) / 9;
+      li[u] = __ldg(M.dom_entry + 3ull * e);
+      lj[u] = __ldg(M.dom_entry + 3ull * e + 1);
+      bi[u] = __ldg(M.dom_entry + 3ull * e + 2);
+    }
+    double v[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const uint32_t t = t0 + u * kInvThreads;
+      v[u] = level_block(M, bi[u])[(t < values ? t : t0) % 9];
+    }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const uint32_t t = t0 + u * kInvThreads;
+      if (t >= values) continue;
+      const int el = (int)(t % 9), k = el / 3, m = el % 3;
+      A[(3 * li[u] + k) * n + 3 * lj[u] + m] = v[u];
+      if (li[u] != lj[u]) A[(3 * lj[u] + m) * n + 3 * li[u] + k] = v[u];
+    }
   }
   __syncthreads();
   // Gauss-Jordan without pivoting (SPD domains): after a step, A holds the
@@ -152,13 +173,13 @@ __global__ void __launch_bounds__(kInvThreads, PB == 2 ? 2 : 1) mas_domain_inver
       const uint32_t i = ty + 16 * a, j = tx + 16 * b;
       R[a][b] = (i < n && j < n) ? A[i * n + j] * dinv[i] * dinv[j] : (i == j && i < np ? 1.0 : 0.0);
     }
-  // PB == 2 runs the symmetric form (the sweep operator): with v = S[:,K]
+  // T <= 6 runs the symmetric form (the sweep operator): with v = S[:,K]
   // except v[K,:] = P - I, the update S -= (v P^-1) v^T and then S[k,k] -= 2
   // on the pivots sweeps K; after every pivot S holds -S_0^-1.  The update is
   // symmetric, so only the upper register tiles (a <= b) are kept: v is read
   // from the published column K for rows in tiles up to the pivot's and from
   // the published row K beyond it, never from a lower tile.
-  constexpr bool kSweep = PB == 2;
+  constexpr bool kSweep = T <= 6;
   // publish block k: colb[buf][i][m] = C[i][m], rowb[buf][m][j] = R[m][j].
   // Block k lies in register column/row KB = PB k / 16 of its owners; KB is a
   // compile-time constant (the step loop is unrolled over it), so the owners
@@ -198,14 +219,13 @@ __global__ void __launch_bounds__(kInvThreads, PB == 2 ? 2 : 1) mas_domain_inver
     if (k >= nblk) break;
     const int buf = (int)(k & 1);
     double P[PB][PB];
-    if constexpr (PB == 2) {
-      const double q00 = colb[buf][(2 * k) * 2] + 1.0, q01 = colb[buf][(2 * k) * 2 + 1];
-      const double q10 = colb[buf][(2 * k + 1) * 2], q11 = colb[buf][(2 * k + 1) * 2 + 1] + 1.0;
-      const double da = q00 * q11 - q01 * q10;
-      const double ida = 1.0 / da;
-      P[0][0] = q11 * ida; P[0][1] = -q01 * ida; P[1][0] = -q10 * ida; P[1][1] = q00 * ida;
-      if (!(q00 > tol && da > tol * q00) && threadIdx.x == 0) bad = 1;
-    } else {
+    // In the symmetric form w = v P^-1 is formed once a row (three warps, a
+    // barrier more a step) instead of by every thread for its six rows: with
+    // four pivots a step the FP64 work a pivot falls from 41 to about 25
+    // instructions a thread, at the same number of barriers a pivot as two
+    // pivots a step with w formed by everyone.
+    const bool mine = !kSweep || threadIdx.x < 16 * T;  // rows past np have v = 0
+    if (mine) {
     // P^-1 of the 4x4 pivot block (every thread alike) by 2x2 blocks:
     // P = [A B; B' D], S = D - B' A^-1 B, P^-1 = [A^-1 + E S^-1 E', -E S^-1;
     // -S^-1 E', S^-1] with E = A^-1 B (P is symmetric up to rounding; the
@@ -240,7 +260,21 @@ __global__ void __launch_bounds__(kInvThreads, PB == 2 ? 2 : 1) mas_domain_inver
       // scalar pivots of the same elimination: q00, da / q00, and the two of S
       const bool ok = q[0][0] > tol && da > tol * q[0][0] && s00 > tol && ds > tol * s00;
       if (!ok && threadIdx.x == 0) bad = 1;
+      if constexpr (kSweep) {
+        const uint32_t i = threadIdx.x;
+        double c[PB];
+#pragma unroll
+        for (int l = 0; l < PB; ++l) c[l] = (int)(i >> 4) <= KB ? colb[buf][i * PB + l] : rowb[buf][l * 128 + i];
+#pragma unroll
+        for (int m = 0; m < PB; ++m) {
+          double acc = 0.0;
+#pragma unroll
+          for (int l = 0; l < PB; ++l) acc += c[l] * P[l][m];
+          wbuf[i * PB + m] = acc;
+        }
+      }
     }
+    if constexpr (kSweep) __syncthreads();
     double rj[PB][T];
 #pragma unroll
     for (int m = 0; m < PB; ++m)
@@ -249,17 +283,21 @@ __global__ void __launch_bounds__(kInvThreads, PB == 2 ? 2 : 1) mas_domain_inver
         rj[m][b] = (!kSweep || b >= KB) ? rowb[buf][m * 128 + tx + 16 * b] : colb[buf][(tx + 16 * b) * PB + m];
 #pragma unroll
     for (int a = 0; a < T; ++a) {
-      double c[PB];
-#pragma unroll
-      for (int l = 0; l < PB; ++l)
-        c[l] = (!kSweep || a <= KB) ? colb[buf][(ty + 16 * a) * PB + l] : rowb[buf][l * 128 + ty + 16 * a];
       double w[PB];
+      if constexpr (kSweep) {
 #pragma unroll
-      for (int m = 0; m < PB; ++m) {
-        double acc = 0.0;
+        for (int m = 0; m < PB; ++m) w[m] = wbuf[(ty + 16 * a) * PB + m];
+      } else {
+        double c[PB];
 #pragma unroll
-        for (int l = 0; l < PB; ++l) acc += c[l] * P[l][m];
-        w[m] = acc;
+        for (int l = 0; l < PB; ++l) c[l] = colb[buf][(ty + 16 * a) * PB + l];
+#pragma unroll
+        for (int m = 0; m < PB; ++m) {
+          double acc = 0.0;
+#pragma unroll
+          for (int l = 0; l < PB; ++l) acc += c[l] * P[l][m];
+          w[m] = acc;
+        }
       }
 #pragma unroll
       for (int b = 0; b < T; ++b) {
@@ -1017,12 +1055,12 @@ int32_t ys_mas_create(const ys_mas_desc* d, void** handle) {
   cudaError_t e = cudaSuccess;
   {
     const size_t smem = sizeof(double) * d->max_domain_dofs * d->max_domain_dofs;
-    e = cudaFuncSetAttribute(ys::mas_domain_inverse<6, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = cudaFuncSetAttribute(ys::mas_domain_inverse<6, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(ys::mas_domain_inverse<8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     // prefer the largest shared-memory carveout so two 96-DoF domains fit per SM
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(ys::mas_domain_inverse<6, 2>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+      e = cudaFuncSetAttribute(ys::mas_domain_inverse<6, 4>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(ys::mas_domain_inverse<8, 4>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   }
@@ -1063,7 +1101,7 @@ int32_t ys_mas_numeric_update(void* handle, const double* fine_values, void* str
   }
   const size_t smem = sizeof(double) * M.max_dofs * M.max_dofs;
   if (M.max_dofs <= 96)
-    ys::mas_domain_inverse<6, 2><<<M.num_domains, ys::kInvThreads, smem, s>>>(M);
+    ys::mas_domain_inverse<6, 4><<<M.num_domains, ys::kInvThreads, smem, s>>>(M);
   else
     ys::mas_domain_inverse<8, 4><<<M.num_domains, ys::kInvThreads, smem, s>>>(M);
   YS_CHECK_LAUNCH();
