@@ -792,6 +792,22 @@ int32_t ys_mas_gemv(void* handle, void* stream, uint64_t* algorithmic_bytes);
  * target slot (repeated slots included); grad_outer[n+1] prefix counts. */
 int32_t ys_gradient_coordinates(const uint32_t* codes, const uint16_t* sizes, uint32_t n, uint32_t K,
                                 uint32_t* grad_outer, uint32_t* coords, uint16_t* dims, void* stream);
+
+/* The index steps with scratch from the caller, for structures that are
+ * rebuilt every step (the forms above draw it from the device's memory pool,
+ * which gives its pages back at every synchronisation).  bytes >=
+ * ys_index_workspace_bytes(n); one scratch serves calls in a row on a stream.
+ * ys_gradient_outer writes the [n + 1] offsets, ys_gradient_fill the
+ * coordinates at them; together they are ys_gradient_coordinates. */
+uint64_t ys_index_workspace_bytes(uint32_t n);
+int32_t ys_compress_indices_ws(const uint32_t* codes, const uint16_t* sizes, uint32_t n, uint32_t K,
+                               int16_t* perm, uint16_t* total_sizes, uint32_t* coord_outer, void* workspace,
+                               uint64_t workspace_bytes, void* stream);
+int32_t ys_gradient_outer(const uint32_t* codes, uint32_t n, uint32_t K, uint32_t* grad_outer, void* workspace,
+                          uint64_t workspace_bytes, void* stream);
+int32_t ys_gradient_fill(const uint32_t* codes, const uint16_t* sizes, uint32_t n, uint32_t K,
+                         const uint32_t* grad_outer, uint32_t* coords, uint16_t* dims, void* stream);
+
 /* ys_assemble specialised for 3x3 blocks.  out32 (when not NULL) receives
  * the FP32 copy in 16-byte aligned slots of 12 floats per block (block u at
  * out32 + 12 u, the last 3 floats unused): the layout ys_spmv3, the tiled

@@ -42,7 +42,7 @@ def test_cube_solutions(side, mixed):
 
 @pytest.mark.parametrize("mixed", [True, False])
 def test_rows_split_over_warps(mixed):
-  cc = scenes.cloth_contact(48, 2000, num_bodies=3, body_subdivisions=4, seed=2)
+  cc = scenes.cloth_contact(56, 1000, spacing=0.025, dhat=1e-2, num_bodies=1, body_subdivisions=4, seed=2)
   sc, _ = scenes.cloth_contact_scene(cc)
   sc.minimizer.setSolver("mas", mixed_spmv=mixed, stop_rule="residual")
   x = np.concatenate([s.cpu().numpy() for s in sc.minimizeEnergy(tolerance=1e-6, maxIterations=5000)])

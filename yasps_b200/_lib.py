@@ -193,6 +193,10 @@ SIGNATURES = {
     "ys_mas_destroy": (i32, [vp]),
     "ys_mas_gemv": (i32, [vp, vp, P(u64)]),
     "ys_gradient_coordinates": (i32, [vp, vp, u32, u32, vp, vp, vp, vp]),
+    "ys_index_workspace_bytes": (u64, [u32]),
+    "ys_compress_indices_ws": (i32, [vp, vp, u32, u32, vp, vp, vp, vp, u64, vp]),
+    "ys_gradient_outer": (i32, [vp, u32, u32, vp, vp, u64, vp]),
+    "ys_gradient_fill": (i32, [vp, vp, u32, u32, vp, vp, vp, vp]),
     "ys_refine_workspace_doubles": (u64, [u32]),
     "ys_refine_residual": (i32, [P(Matrix3), vp, vp, vp, vp, vp, P(f64), vp]),
     "ys_serve_workspace_doubles": (u64, [u32]),

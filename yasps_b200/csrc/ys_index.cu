@@ -299,6 +299,55 @@ int32_t ys_gradient_coordinates(const uint32_t* codes, const uint16_t* sizes, ui
   return YS_OK;
 }
 
+// Bytes of CUB's inclusive scan of n counts (ys_index_workspace_bytes).
+static cudaError_t count_scan(void* tmp, size_t& bytes, uint32_t* counts, uint32_t n, cudaStream_t s) {
+  return cub::DeviceScan::InclusiveSum(tmp, bytes, counts, counts, (int)n, s);
+}
+
+uint64_t ys_index_workspace_bytes(uint32_t n) {
+  size_t bytes = 0;
+  if (n == 0 || count_scan(nullptr, bytes, nullptr, n, nullptr) != cudaSuccess) return 16;
+  return bytes > 16 ? bytes : 16;
+}
+
+int32_t ys_gradient_outer(const uint32_t* codes, uint32_t n, uint32_t K, uint32_t* grad_outer, void* workspace,
+                          uint64_t workspace_bytes, void* stream) {
+  cudaStream_t s = (cudaStream_t)stream;
+  YS_CUDA_TRY(cudaMemsetAsync(grad_outer, 0, sizeof(uint32_t), s));
+  if (n == 0) return YS_OK;
+  YS_REQUIRE(workspace && workspace_bytes >= ys_index_workspace_bytes(n), YS_ERR_CAPACITY, "index workspace too small");
+  ys::grad_count_kernel<<<ys::grid_for(n, 256), 256, 0, s>>>(codes, n, K, grad_outer + 1);
+  YS_CHECK_LAUNCH();
+  size_t bytes = (size_t)workspace_bytes;
+  YS_CUDA_TRY(count_scan(workspace, bytes, grad_outer + 1, n, s));
+  return YS_OK;
+}
+
+int32_t ys_gradient_fill(const uint32_t* codes, const uint16_t* sizes, uint32_t n, uint32_t K,
+                         const uint32_t* grad_outer, uint32_t* coords, uint16_t* dims, void* stream) {
+  YS_REQUIRE(grad_outer && coords && dims, YS_ERR_INVALID, "null argument");
+  if (n == 0) return YS_OK;
+  ys::grad_coords_kernel<<<ys::grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(codes, sizes, n, K, grad_outer,
+                                                                                 coords, dims);
+  YS_CHECK_LAUNCH();
+  return YS_OK;
+}
+
+int32_t ys_compress_indices_ws(const uint32_t* codes, const uint16_t* sizes, uint32_t n, uint32_t K, int16_t* perm,
+                               uint16_t* total_sizes, uint32_t* coord_outer, void* workspace,
+                               uint64_t workspace_bytes, void* stream) {
+  YS_REQUIRE(K >= 1 && K <= 4096, YS_ERR_INVALID, "K must be 1..4096");
+  cudaStream_t s = (cudaStream_t)stream;
+  YS_CUDA_TRY(cudaMemsetAsync(coord_outer, 0, sizeof(uint32_t), s));
+  if (n == 0) return YS_OK;
+  YS_REQUIRE(workspace && workspace_bytes >= ys_index_workspace_bytes(n), YS_ERR_CAPACITY, "index workspace too small");
+  ys::compress_kernel<<<ys::grid_for(n, 256), 256, 0, s>>>(codes, sizes, n, K, perm, total_sizes, coord_outer + 1);
+  YS_CHECK_LAUNCH();
+  size_t bytes = (size_t)workspace_bytes;
+  YS_CUDA_TRY(count_scan(workspace, bytes, coord_outer + 1, n, s));
+  return YS_OK;
+}
+
 const char* ys_last_error(void) { return g_last_error.c_str(); }
 
 int32_t ys_version(void) { return 100; }

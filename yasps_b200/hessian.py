@@ -491,15 +491,18 @@ class hessian:
     torch = _torch()
     s = L.stream_ptr()
     info = []
-    total = 0
+    work, nbytes = self._index_scratch(max((t.n for t in terms), default=0))
     for t in terms:
       n = t.n
       codes, sizes, K, stride = t.codes()
       perm = torch.empty(max(n * K, 1), dtype=torch.int16, device=_dev())
       outer = torch.empty(n + 1, dtype=torch.int32, device=_dev())
-      L.call("ys_compress_indices", L.ptr(codes), L.ptr(sizes), n, K, L.ptr(perm), None, L.ptr(outer), s)
-      m = int(outer[n].item()) if n else 0
-      info.append(dict(term=t, codes=codes, sizes=sizes, K=K, stride=stride, perm=perm, outer=outer, m=m, off=total))
+      L.call("ys_compress_indices_ws", L.ptr(codes), L.ptr(sizes), n, K, L.ptr(perm), None, L.ptr(outer),
+             L.ptr(work), nbytes, s)
+      info.append(dict(term=t, codes=codes, sizes=sizes, K=K, stride=stride, perm=perm, outer=outer))
+    total = 0
+    for d, m in zip(info, self._last_counts([d["outer"] for d in info])):
+      d["m"], d["off"] = m, total
       total += m
     coords = torch.empty(max(2 * total, 2), dtype=torch.int32, device=_dev())
     dims = torch.empty(max(2 * total, 2), dtype=torch.int16, device=_dev())
@@ -511,26 +514,42 @@ class hessian:
              d["term"].n, d["K"], coords.data_ptr() + 8 * off, dims.data_ptr() + 4 * off, s)
     return info, coords, dims, total
 
+  @staticmethod
+  def _index_scratch(n: int):
+    """Scratch of the index steps for up to ``n`` instances (stream-ordered
+    caching allocator: no pool is trimmed and grown again between steps)."""
+    torch = _torch()
+    nbytes = int(L.load().ys_index_workspace_bytes(int(n)))
+    return torch.empty(nbytes, dtype=torch.uint8, device=_dev()), nbytes
+
+  @staticmethod
+  def _last_counts(outers) -> list:
+    """Totals (last entries) of the offset arrays, in one device read."""
+    if not outers:
+      return []
+    return _torch().cat([o[-1:] for o in outers]).cpu().tolist()
+
   def _gradient_plan(self, infos):
     torch = _torch()
     s = L.stream_ptr()
-    total = 0
-    for d in infos:
+    work, nbytes = self._index_scratch(max((d["term"].n for d in infos), default=0))
+    fresh = [d for d in infos if "gouter" not in d]  # (the static terms' offsets stay)
+    for d in fresh:
       n, K = d["term"].n, d["K"]
       d["gouter"] = torch.empty(n + 1, dtype=torch.int32, device=_dev())
-      L.call("ys_gradient_coordinates", L.ptr(d["codes"]), L.ptr(d["sizes"]), n, K, L.ptr(d["gouter"]), None, None,
-             None, s)
-      d["gm"] = int(d["gouter"][n].item()) if n else 0
+      L.call("ys_gradient_outer", L.ptr(d["codes"]), n, K, L.ptr(d["gouter"]), L.ptr(work), nbytes, s)
+    for d, m in zip(fresh, self._last_counts([d["gouter"] for d in fresh])):
+      d["gm"] = m
+    total = 0
+    for d in infos:
       d["goff"] = total
       total += d["gm"]
     coords = torch.empty(max(2 * total, 2), dtype=torch.int32, device=_dev())
     dims = torch.empty(max(2 * total, 2), dtype=torch.int16, device=_dev())
     for d in infos:
-      if d["gm"] == 0:
-        continue
-      n, K = d["term"].n, d["K"]
-      L.call("ys_gradient_coordinates", L.ptr(d["codes"]), L.ptr(d["sizes"]), n, K, L.ptr(d["gouter"]),
-             coords.data_ptr() + 8 * d["goff"], dims.data_ptr() + 4 * d["goff"], s)
+      if d["gm"]:
+        L.call("ys_gradient_fill", L.ptr(d["codes"]), L.ptr(d["sizes"]), d["term"].n, d["K"], L.ptr(d["gouter"]),
+               coords.data_ptr() + 8 * d["goff"], dims.data_ptr() + 4 * d["goff"], s)
     pat = _Pattern(coords, dims, total)
     self._grad_pattern = pat
     self._grad_records = torch.empty(max(pat.total_records, 1), dtype=torch.float64, device=_dev())
