@@ -37,6 +37,7 @@ constexpr int kLoopThreads = 512;
 constexpr uint32_t kLoopCoarse = 512;    // most nodes of the levels from 2 on (their residuals in shared memory)
 constexpr uint32_t kLongRow = 64;        // longer rows are split over warps of the whole grid
 constexpr uint32_t kLongSegment = 128;   // entries a warp takes of a long row
+constexpr uint32_t kLoopGroup = 12;      // more level-2 domains than this go three to a CTA
 constexpr int kLoopMaxDofs = 4;          // 3-DoF entries a lane holds of a domain of at most 128 DoF
 
 struct LoopParams {
@@ -712,19 +713,29 @@ __global__ void __launch_bounds__(kLoopThreads, 1) mas_pcg_loop(const __grid_con
     const uint32_t first2 = M.levels > 2 ? P.level_domain[2] : M.num_domains;
     const uint32_t first1 = M.levels > 1 ? P.level_domain[1] : M.num_domains, n1 = first2 - first1;
     const uint32_t whole = WIDE ? M.num_domains : M.num_domains - first2;  // domains by whole CTAs, from the last
-    // the other CTAs share the rest, a warp a domain, when there are enough
-    const uint32_t skip = !WIDE && whole < gridDim.x / 2 ? whole : 0;
+    // of those, a CTA takes one of the levels >= 3 (their residuals are a chain
+    // of sums) and one of level 2, or three of many: 18 level-2 domains then
+    // leave 12 CTAs more to the fine levels (65,600 variables, cloth with
+    // bodies: 15.7 -> 14.0 ms a step in FP32, 16.4 -> 15.0 in FP64), where the
+    // few of a cube would only wait for one another.  The line at 12 lies
+    // between the two kinds, not at a measured crossing.
+    // The other CTAs share the rest, a warp a domain, when there are enough.
+    const uint32_t n3 = !WIDE && M.levels > 3 ? M.num_domains - P.level_domain[3] : 0;
+    const uint32_t n2 = WIDE ? 0 : whole - n3, nb2 = n2 > kLoopGroup ? (n2 + 2) / 3 : n2;
+    const uint32_t skip = !WIDE && n3 + nb2 < gridDim.x / 2 ? n3 + nb2 : 0;
+    const uint32_t whole_end = skip && blockIdx.x >= skip ? 0 : whole;
+    const uint32_t whole_step = !skip ? gridDim.x : (blockIdx.x < n3 ? whole : nb2);
     const uint32_t workers = gridDim.x - skip;
     uint32_t job = first2;
     if (!WIDE && warp < (int)P.gemv_warps && blockIdx.x >= skip) job = warp * workers + (blockIdx.x - skip);
     LoopTilesAhead ahead;
-    if (blockIdx.x < whole) loop_prefetch(M, M.num_domains - 1 - blockIdx.x, ahead.t[0]);
+    if (blockIdx.x < whole_end) loop_prefetch(M, M.num_domains - 1 - blockIdx.x, ahead.t[0]);
     else if (job < first2) ahead.first(M, job < n1 ? first1 + job : job - n1);
     if (!loop_barrier(P, S)) break;
     // C
     acc = 0.0;
     {
-      for (uint32_t k = blockIdx.x; k < whole; k += gridDim.x) {
+      for (uint32_t k = blockIdx.x; k < whole_end; k += whole_step) {
         const uint32_t d = M.num_domains - 1 - k;
         uint32_t l = 0;
         while (l + 1 < M.levels && d >= P.level_domain[l + 1]) ++l;
@@ -739,7 +750,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) mas_pcg_loop(const __grid_con
       }
       if constexpr (!WIDE) {
         float4* const area = loop_areas + (size_t)warp * P.area;
-        const bool fresh = blockIdx.x >= whole;  // `ahead` still holds the first job's tiles
+        const bool fresh = blockIdx.x >= whole_end;  // `ahead` still holds the first job's tiles
         for (uint32_t j = job; j < first2; j += P.gemv_warps * workers) {
           const bool one = j < n1;  // the level-1 domains first
           const uint32_t d = one ? first1 + j : j - n1;
