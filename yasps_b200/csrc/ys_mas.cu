@@ -924,56 +924,39 @@ static cudaError_t add_loop_kernel(cudaGraph_t body, cudaGraphNode_t* node, Loop
   return e;
 }
 
-// The loop's own device memory: the segments of the rows longer than kLongRow
-// (from the row pointers), the grid's partial sums (a CTA an SM at most, more
-// than the workspace of a tiny system holds) and the wide form's corrections.
-static cudaError_t loop_memory(LoopParams& L, uint32_t nv, bool wide, unsigned max_grid, void** owned) {
-  std::vector<std::vector<uint32_t>> rp(L.nsets, std::vector<uint32_t>(nv + 1));
-  for (int s = 0; s < L.nsets; ++s) {
-    const cudaError_t e =
-        cudaMemcpy(rp[s].data(), L.sets[s].row_ptr, sizeof(uint32_t) * (nv + 1), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return e;
-  }
-  std::vector<uint4> seg;
-  std::vector<uint32_t> row, first;
-  for (uint32_t i = 0; i < nv; ++i) {
-    const size_t before = seg.size();
-    for (int s = 0; s < L.nsets; ++s) {
-      const uint32_t e0 = rp[s][i], e1 = rp[s][i + 1];
-      if (e1 - e0 <= kLongRow) continue;
-      for (uint32_t e = e0; e < e1; e += kLongSegment)
-        seg.push_back(make_uint4(i, e, std::min(e1, e + kLongSegment), (uint32_t)s));
-    }
-    if (seg.size() > before) {
-      row.push_back(i);
-      first.push_back((uint32_t)before);
-    }
-  }
-  L.num_segments = (uint32_t)seg.size();
-  L.num_long = (uint32_t)row.size();
-  first.push_back(L.num_segments);
-  const size_t b0 = sizeof(uint4) * seg.size(), b1 = sizeof(double) * 3 * seg.size();
-  const size_t b2 = sizeof(uint32_t) * row.size(), b3 = sizeof(uint32_t) * first.size();
-  const size_t bz = wide ? sizeof(double) * 3 * L.M.packed_nodes : 0;
-  const size_t bp = sizeof(double) * 3 * max_grid;  // p.q, r.z and r.r of every CTA
-  char* dev = nullptr;
-  cudaError_t e = cudaMalloc(&dev, bp + bz + 16 + b0 + b1 + b2 + b3);
-  if (e != cudaSuccess) return e;
-  *owned = dev;
-  L.partials = reinterpret_cast<double*>(dev);
-  L.zl64 = reinterpret_cast<double*>(dev + bp);
-  dev += (bp + bz + 15) / 16 * 16;
-  L.segments = reinterpret_cast<const uint4*>(dev);
-  L.seg = reinterpret_cast<double*>(dev + b0);
-  L.long_row = reinterpret_cast<const uint32_t*>(dev + b0 + b1);
-  L.long_first = reinterpret_cast<const uint32_t*>(dev + b0 + b1 + b2);
-  if (b0) e = cudaMemcpy(dev, seg.data(), b0, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && b2) e = cudaMemcpy(dev + b0 + b1, row.data(), b2, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(dev + b0 + b1 + b2, first.data(), b3, cudaMemcpyHostToDevice);
-  return e;
+// The loop's part of the solve's workspace (after 16-byte alignment).  The
+// partials take p.q, r.z and r.r of every CTA.  A system of at most
+// kLoopMaxGrid domains may run the wide form, whose FP64 corrections are one
+// per packed node: every node lies in one domain of its level.
+constexpr uint32_t kLoopMaxGrid = 256;
+
+static uint32_t loop_max_segments(uint32_t nv) { return nv / 4 + 1024; }
+
+static uint64_t loop_wide_nodes(uint32_t nv) {
+  return std::min<uint64_t>((uint64_t)kMaxLevels * nv, (uint64_t)kLoopMaxGrid * (128 / 3));
 }
 
-cudaError_t mas_add_loop_node(void* mas, cudaGraph_t body, MasPcgHooks* hooks, bool* used) {
+uint64_t mas_loop_workspace_doubles(uint32_t nv) {
+  if (nv > kLoopMaxVars) return 0;
+  const uint64_t seg = loop_max_segments(nv);
+  return 2 + 2 * seg + sizeof(LoopTable) / 8 + 1 + 3ull * kLoopMaxGrid + 3 * seg + 3 * loop_wide_nodes(nv) + seg + 1;
+}
+
+static void loop_memory(LoopParams& L, uint32_t nv, double* w) {
+  if (reinterpret_cast<uintptr_t>(w) % 16) ++w;
+  const uint64_t seg = loop_max_segments(nv);
+  L.max_segments = (uint32_t)seg;
+  L.segments = reinterpret_cast<uint4*>(w); w += 2 * seg;
+  L.table = reinterpret_cast<LoopTable*>(w); w += sizeof(LoopTable) / 8 + 1;
+  L.partials = w; w += 3ull * kLoopMaxGrid;
+  L.seg = w; w += 3 * seg;
+  L.zl64 = w; w += 3 * loop_wide_nodes(nv);
+  L.long_row = reinterpret_cast<uint32_t*>(w);
+  L.long_first = L.long_row + seg;
+}
+
+cudaError_t mas_add_loop_node(void* mas, cudaGraph_t g, cudaGraph_t body, cudaGraphNode_t* tables,
+                              MasPcgHooks* hooks, bool* used) {
   *used = false;
   auto* h = static_cast<MasHandle*>(mas);
   auto* P = static_cast<MasPcg*>(hooks->params);
@@ -984,11 +967,6 @@ cudaError_t mas_add_loop_node(void* mas, cudaGraph_t body, MasPcgHooks* hooks, b
   for (int s = 0; s < P->nsets; ++s) L.sets[s] = P->sets[s];
   L.nsets = P->nsets;
   L.M = M;
-  std::vector<uint32_t> ptr(M.num_domains + 1);
-  cudaError_t e = cudaMemcpy(ptr.data(), M.dom_node_ptr, sizeof(uint32_t) * ptr.size(), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return e;
-  for (uint32_t l = 0; l <= M.levels; ++l)
-    L.level_domain[l] = (uint32_t)(std::lower_bound(ptr.begin(), ptr.end(), M.level_node_offset[l]) - ptr.begin());
   L.x = P->x;
   L.r = P->r;
   L.p = P->p;
@@ -1000,19 +978,23 @@ cudaError_t mas_add_loop_node(void* mas, cudaGraph_t body, MasPcgHooks* hooks, b
   L.area = (uint32_t)(gemv_smem_bytes(M.max_dofs) / 16);
   L.cond = P->cond;
   int dev = 0, sms = 0, coop = 0;
-  e = cudaGetDevice(&dev);
+  cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess || !coop) return e;
-  const bool wide = M.num_domains <= (uint32_t)sms;
-  e = loop_memory(L, P->nv, wide, (unsigned)sms, &hooks->owned);
+  sms = std::min(sms, (int)kLoopMaxGrid);
+  const bool wide = M.num_domains <= (uint32_t)sms && M.packed_nodes <= loop_wide_nodes(P->nv);
+  loop_memory(L, P->nv, hooks->loop_workspace);
   cudaGraphNode_t node = nullptr;
-  if (e != cudaSuccess) return e;
   if (wide)
-    return P->fp32 ? add_loop_kernel<float, true>(body, &node, L, P->nv, sms, used)
-                   : add_loop_kernel<double, true>(body, &node, L, P->nv, sms, used);
-  return P->fp32 ? add_loop_kernel<float, false>(body, &node, L, P->nv, sms, used)
-                 : add_loop_kernel<double, false>(body, &node, L, P->nv, sms, used);
+    e = P->fp32 ? add_loop_kernel<float, true>(body, &node, L, P->nv, sms, used)
+                : add_loop_kernel<double, true>(body, &node, L, P->nv, sms, used);
+  else
+    e = P->fp32 ? add_loop_kernel<float, false>(body, &node, L, P->nv, sms, used)
+                : add_loop_kernel<double, false>(body, &node, L, P->nv, sms, used);
+  if (e != cudaSuccess || !*used) return e;
+  void* args[] = {&L};
+  return add_kernel(g, tables, nullptr, 0, (const void*)loop_tables_kernel, 1, kTableThreads, 0, args);
 }
 
 }  // namespace ys

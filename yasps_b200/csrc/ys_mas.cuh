@@ -8,7 +8,7 @@ namespace ys {
 struct MasPcgHooks {
   void* params = nullptr;  // owned by the MAS handle
   bool fused_direction = false;  // the loop body's last MAS node also updates p
-  void* owned = nullptr;         // device memory of mas_add_loop_node (freed with the PCG handle)
+  double* loop_workspace = nullptr;  // mas_loop_workspace_doubles(num_vars) of the caller's workspace
 };
 
 // Nodes computing r = g - H x (or r = g), z = M^-1 r, p = z and the initial
@@ -26,7 +26,12 @@ cudaError_t mas_add_update_nodes(void* mas, cudaGraph_t body, const cudaGraphNod
                                  cudaGraphNode_t* last, MasPcgHooks* hooks);
 
 // The whole loop as one cooperative kernel, the body's only node, when the
-// system is small enough for it (*used).
-cudaError_t mas_add_loop_node(void* mas, cudaGraph_t body, MasPcgHooks* hooks, bool* used);
+// system is small enough for it (*used).  *tables is then the node of `g` that
+// reads the row plan for it: the loop has to come after it.
+cudaError_t mas_add_loop_node(void* mas, cudaGraph_t g, cudaGraph_t body, cudaGraphNode_t* tables,
+                              MasPcgHooks* hooks, bool* used);
+
+// Doubles of the solve's workspace that the one-kernel loop takes (0 beyond its sizes).
+uint64_t mas_loop_workspace_doubles(uint32_t num_vars);
 
 }  // namespace ys

@@ -24,6 +24,12 @@
 // third to a sixth of the iterations (336 against 1862 on 70 vertices with
 // stiff friction), and a domain a CTA costs no more than in FP32.
 //
+// Rows longer than a threshold are split into segments over the warps of the
+// whole grid.  Their table is a node of the solve's graph (loop_tables_kernel,
+// beside the nodes that form the first residual), so it follows the row plan
+// that stands in the caller's buffers at each launch, as every other read of
+// the plan does.
+//
 // Barrier waits are bounded (kPollLimitParam polls): a CTA that gives up marks
 // the solve void (kBarrierFail) and every CTA leaves.
 #pragma once
@@ -35,16 +41,22 @@ namespace ys {
 
 constexpr int kLoopThreads = 512;
 constexpr uint32_t kLoopCoarse = 512;    // most nodes of the levels from 2 on (their residuals in shared memory)
-constexpr uint32_t kLongRow = 64;        // longer rows are split over warps of the whole grid
-constexpr uint32_t kLongSegment = 128;   // entries a warp takes of a long row
+constexpr uint32_t kLongRow = 64;        // longer rows are split over warps, in segments of twice that
 constexpr uint32_t kLoopGroup = 12;      // more level-2 domains than this go three to a CTA
 constexpr int kLoopMaxDofs = 4;          // 3-DoF entries a lane holds of a domain of at most 128 DoF
+
+// What the loop needs to know of the row plan and of the domains; written by
+// loop_tables_kernel at every launch.
+struct LoopTable {
+  uint32_t threshold;      // longer rows (per block set) are split
+  uint32_t num_segments, num_long;
+  uint32_t level_domain[kMaxLevels + 1];  // first domain of each level
+};
 
 struct LoopParams {
   SpmvSet sets[2];
   int nsets;
   MasDev M;
-  uint32_t level_domain[kMaxLevels + 1];  // first domain of each level
   double* x;
   double* r;
   double* p;
@@ -58,10 +70,11 @@ struct LoopParams {
   uint32_t area;           // float4 of one area
   // long rows: segments (row, first entry, last entry, set) ordered by row and
   // set; long_row lists the rows, long_first their first segments
-  const uint4* segments;
-  const uint32_t* long_row;
-  const uint32_t* long_first;
-  uint32_t num_segments, num_long;
+  LoopTable* table;
+  uint4* segments;
+  uint32_t* long_row;
+  uint32_t* long_first;
+  uint32_t max_segments;   // room in segments, long_row and seg
   double* seg;             // 3 per segment
   double* zl64;            // the wide form's FP64 level corrections, 3 per packed node
   cudaGraphConditionalHandle cond;
@@ -97,6 +110,7 @@ struct LoopState {
   double delta, prev, rr, curv, alpha, beta, it;
   unsigned long long target;
   int status, ok;
+  LoopTable t;
 };
 
 // Bounded grid barrier on a monotonic arrival count; false: gave up.
@@ -141,10 +155,11 @@ __device__ __forceinline__ double loop_total(const double* partials) {
 
 // The long rows' segments, a warp each; returns the lane's share of p.q.
 template <typename T>
-__device__ __forceinline__ double loop_segments(const LoopParams& P, const typename LoopTypes<T>::X* px) {
+__device__ __forceinline__ double loop_segments(const LoopParams& P, const LoopState& L,
+                                                const typename LoopTypes<T>::X* px) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double dot = 0.0;
-  for (uint32_t s = warp * gridDim.x + blockIdx.x; s < P.num_segments; s += (kLoopThreads / 32) * gridDim.x) {
+  for (uint32_t s = warp * gridDim.x + blockIdx.x; s < L.t.num_segments; s += (kLoopThreads / 32) * gridDim.x) {
     const uint4 it = __ldg(P.segments + s);
     const SpmvSet& S = P.sets[it.w];
     const T* vals = set_values(S, T(0));
@@ -181,7 +196,8 @@ struct LoopRows {
   uint32_t e0[U], e1[U];
   uint32_t eb[U][2], col[U][2];
 
-  __device__ __forceinline__ void bounds(const LoopParams& P, uint32_t base, uint32_t r1) {
+  __device__ __forceinline__ void bounds(const LoopParams& P, const LoopState& L, uint32_t base,
+                                         uint32_t r1) {
     const SpmvSet& S = P.sets[0];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -189,7 +205,7 @@ struct LoopRows {
       const bool valid = i < r1;
       e0[u] = valid ? __ldg(S.row_ptr + i) : 0u;
       e1[u] = valid ? __ldg(S.row_ptr + i + 1) : 0u;
-      if (e1[u] - e0[u] > kLongRow) e1[u] = e0[u];
+      if (e1[u] - e0[u] > L.t.threshold) e1[u] = e0[u];
     }
   }
   __device__ __forceinline__ void indices(const LoopParams& P, int sub) {
@@ -210,8 +226,9 @@ struct LoopRows {
 // of p.q.  R holds the first round's rows on entry and the first round's again
 // on exit.
 template <typename T, int U>
-__device__ __forceinline__ double loop_spmv(const LoopParams& P, const typename LoopTypes<T>::X* px,
-                                            LoopRows<T, U>& R, uint32_t first, uint32_t r1) {
+__device__ __forceinline__ double loop_spmv(const LoopParams& P, const LoopState& L,
+                                            const typename LoopTypes<T>::X* px, LoopRows<T, U>& R, uint32_t first,
+                                            uint32_t r1) {
   constexpr uint32_t kRows = kLoopThreads / 8;
   const int sub = threadIdx.x & 7;
   const SpmvSet& S = P.sets[0];
@@ -246,7 +263,7 @@ __device__ __forceinline__ double loop_spmv(const LoopParams& P, const typename 
       }
       // the next round's rows (the first round's after the last)
       const bool more = wb + U * kRows < r1;
-      R.bounds(P, more ? base + U * kRows : first, r1);
+      R.bounds(P, L, more ? base + U * kRows : first, r1);
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         a[u][0] = a[u][1] = a[u][2] = 0;
@@ -291,8 +308,8 @@ __device__ __forceinline__ double loop_spmv(const LoopParams& P, const typename 
 
 // The same over two block sets (a static and a dynamic one), a row at a time.
 template <typename T>
-__device__ __forceinline__ double loop_spmv_sets(const LoopParams& P, const typename LoopTypes<T>::X* px,
-                                                 uint32_t first, uint32_t r1) {
+__device__ __forceinline__ double loop_spmv_sets(const LoopParams& P, const LoopState& L,
+                                                 const typename LoopTypes<T>::X* px, uint32_t first, uint32_t r1) {
   const int sub = threadIdx.x & 7;
   double dot = 0.0;
   const uint32_t in_warp = (threadIdx.x & 31) >> 3;
@@ -304,7 +321,7 @@ __device__ __forceinline__ double loop_spmv_sets(const LoopParams& P, const type
       const SpmvSet& S = P.sets[s];
       const T* vals = set_values(S, T(0));
       const uint32_t e0 = valid ? __ldg(S.row_ptr + i) : 0u, end = valid ? __ldg(S.row_ptr + i + 1) : 0u;
-      const uint32_t e1 = end - e0 > kLongRow ? e0 : end;
+      const uint32_t e1 = end - e0 > L.t.threshold ? e0 : end;
       T a[3] = {0, 0, 0};
       for (uint32_t e = e0 + sub; e < e1; e += kRowLanes) {
         const uint32_t eb = __ldg(S.entry_block + e), j = __ldg(S.entry_col + e);
@@ -336,7 +353,7 @@ __device__ __forceinline__ double loop_spmv_sets(const LoopParams& P, const type
 // not wait for alpha.
 struct LoopUpdate {
   double q[3], p[3], x[3], r[3];
-  __device__ __forceinline__ void load(const LoopParams& P, uint32_t i) {
+  __device__ __forceinline__ void load(const LoopParams& P, const LoopState& L, uint32_t i) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       q[k] = P.q[3ull * i + k];
@@ -344,12 +361,12 @@ struct LoopUpdate {
       x[k] = P.x[3ull * i + k];
       r[k] = P.r[3ull * i + k];
     }
-    if (P.num_long) {
+    if (L.t.num_long) {
       bool is_long = false;
       for (int s = 0; s < P.nsets; ++s)
-        is_long |= __ldg(P.sets[s].row_ptr + i + 1) - __ldg(P.sets[s].row_ptr + i) > kLongRow;
+        is_long |= __ldg(P.sets[s].row_ptr + i + 1) - __ldg(P.sets[s].row_ptr + i) > L.t.threshold;
       if (is_long) {
-        uint32_t lo = 0, hi = P.num_long;  // long_row is ascending
+        uint32_t lo = 0, hi = L.t.num_long;  // long_row is ascending
         while (hi - lo > 1) {
           const uint32_t mid = (lo + hi) / 2;
           if (__ldg(P.long_row + mid) <= i) lo = mid;
@@ -613,7 +630,9 @@ __global__ void __launch_bounds__(kLoopThreads, 1) mas_pcg_loop(const __grid_con
     S.curv = S.alpha = S.beta = 0.0;
     S.target = 0ull;
     S.status = (int)st[kStatus];
+    S.t = *P.table;
   }
+  __syncthreads();
   // this CTA's rows
   const uint32_t per = ((M.nv + gridDim.x - 1) / gridDim.x + 3u) & ~3u;
   const uint32_t r1 = min(M.nv, (blockIdx.x + 1) * per);
@@ -621,16 +640,16 @@ __global__ void __launch_bounds__(kLoopThreads, 1) mas_pcg_loop(const __grid_con
   constexpr int U = 1;  // 2 spilled registers: slower
   LoopRows<T, U> rows;
   if (P.nsets == 1) {
-    rows.bounds(P, first_row, r1);
+    rows.bounds(P, S, first_row, r1);
     rows.indices(P, threadIdx.x & 7);
   }
   __syncthreads();
   while (S.status == kContinue) {
     // A
     {
-      double dot = P.nsets == 1 ? loop_spmv<T, U>(P, px, rows, first_row, r1)
-                                : loop_spmv_sets<T>(P, px, first_row, r1);
-      if (P.num_segments) dot += loop_segments<T>(P, px);
+      double dot = P.nsets == 1 ? loop_spmv<T, U>(P, S, px, rows, first_row, r1)
+                                : loop_spmv_sets<T>(P, S, px, first_row, r1);
+      if (S.t.num_segments) dot += loop_segments<T>(P, S, px);
       const double s = block_sum<kLoopThreads>(dot, red);
       if (threadIdx.x == 0) P.partials[blockIdx.x] = s;
     }
@@ -651,7 +670,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) mas_pcg_loop(const __grid_con
       up_i = blockIdx.x * kLoopThreads + threadIdx.x;
       up_on = up_i < M.nv;
     }
-    if (up_on) up.load(P, up_i);
+    if (up_on) up.load(P, S, up_i);
     const double curv = loop_total(P.partials), prev = S.delta;
     const bool restart = isfinite(curv) && curv <= 0.0 && isfinite(prev) && prev > 0.0;
     if (!restart && (!isfinite(curv) || curv <= 0.0)) {
@@ -680,7 +699,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) mas_pcg_loop(const __grid_con
             up_on = up_q < up_end;
             if (up_on) {
               up_i = __ldg(M.child_fine + up_q);
-              up.load(P, up_i);
+              up.load(P, S, up_i);
             }
           }
 #pragma unroll
@@ -693,7 +712,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) mas_pcg_loop(const __grid_con
             up_on = up_q < up_end;
             if (up_on) {
               up_i = __ldg(M.child_fine + up_q);
-              up.load(P, up_i);
+              up.load(P, S, up_i);
             }
           }
         }
@@ -702,7 +721,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) mas_pcg_loop(const __grid_con
           acc += up.store(P, up_i, alpha);
           up_i += gridDim.x * kLoopThreads;
           up_on = up_i < M.nv;
-          if (up_on) up.load(P, up_i);
+          if (up_on) up.load(P, S, up_i);
         }
       }
       const double s = block_sum<kLoopThreads>(acc, red);
@@ -710,8 +729,8 @@ __global__ void __launch_bounds__(kLoopThreads, 1) mas_pcg_loop(const __grid_con
     }
     // the first tiles of the warp's (or CTA's) first domain are on their way
     // over the barrier; the coarsest domains go to the first CTAs
-    const uint32_t first2 = M.levels > 2 ? P.level_domain[2] : M.num_domains;
-    const uint32_t first1 = M.levels > 1 ? P.level_domain[1] : M.num_domains, n1 = first2 - first1;
+    const uint32_t first2 = M.levels > 2 ? S.t.level_domain[2] : M.num_domains;
+    const uint32_t first1 = M.levels > 1 ? S.t.level_domain[1] : M.num_domains, n1 = first2 - first1;
     const uint32_t whole = WIDE ? M.num_domains : M.num_domains - first2;  // domains by whole CTAs, from the last
     // of those, a CTA takes one of the levels >= 3 (their residuals are a chain
     // of sums) and one of level 2, or three of many: 18 level-2 domains then
@@ -720,7 +739,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) mas_pcg_loop(const __grid_con
     // few of a cube would only wait for one another.  The line at 12 lies
     // between the two kinds, not at a measured crossing.
     // The other CTAs share the rest, a warp a domain, when there are enough.
-    const uint32_t n3 = !WIDE && M.levels > 3 ? M.num_domains - P.level_domain[3] : 0;
+    const uint32_t n3 = !WIDE && M.levels > 3 ? M.num_domains - S.t.level_domain[3] : 0;
     const uint32_t n2 = WIDE ? 0 : whole - n3, nb2 = n2 > kLoopGroup ? (n2 + 2) / 3 : n2;
     const uint32_t skip = !WIDE && n3 + nb2 < gridDim.x / 2 ? n3 + nb2 : 0;
     const uint32_t whole_end = skip && blockIdx.x >= skip ? 0 : whole;
@@ -738,7 +757,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) mas_pcg_loop(const __grid_con
       for (uint32_t k = blockIdx.x; k < whole_end; k += whole_step) {
         const uint32_t d = M.num_domains - 1 - k;
         uint32_t l = 0;
-        while (l + 1 < M.levels && d >= P.level_domain[l + 1]) ++l;
+        while (l + 1 < M.levels && d >= S.t.level_domain[l + 1]) ++l;
         if (k != blockIdx.x) loop_prefetch(M, d, ahead.t[0]);
         if (l >= 2) loop_coarse(P, d, l, coarse);
         const double* res = l >= 2 ? coarse : (l == 1 ? M.rl64 : P.r);
@@ -825,6 +844,115 @@ __global__ void __launch_bounds__(kLoopThreads, 1) mas_pcg_loop(const __grid_con
     st[kIter] = S.it;
     st[kStatus] = (double)S.status;
     cudaGraphSetConditional(P.cond, 0u);
+  }
+}
+
+// The table of the long rows (and of the levels' domains) from the row plan as
+// it stands: one CTA, a contiguous run of rows a thread, so that the segments
+// are ordered by row whatever the counts are.  It runs beside the nodes that
+// form the first residual, off the solve's critical path.  Where a plan has
+// more segments than there is room for, the threshold and the segments double
+// until they fit (in the end no row is split).
+constexpr int kTableThreads = 1024;
+
+__global__ void __launch_bounds__(kTableThreads) loop_tables_kernel(const __grid_constant__ LoopParams P) {
+  __shared__ uint32_t scan[2][kTableThreads / 32];
+  const MasDev& M = P.M;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t per = (M.nv + kTableThreads - 1) / kTableThreads;
+  const uint32_t r0 = min(M.nv, threadIdx.x * per), r1 = min(M.nv, r0 + per);
+  uint32_t threshold = kLongRow, longs, segs, before_longs, before_segs, all_longs, all_segs;
+  while (true) {
+    longs = segs = 0;
+#pragma unroll 4
+    for (uint32_t i = r0; i < r1; ++i) {
+      uint32_t n = 0;
+      for (int s = 0; s < P.nsets; ++s) {
+        const uint32_t len = P.sets[s].row_ptr[i + 1] - P.sets[s].row_ptr[i];
+        if (len > threshold) n += (len - 1) / (2 * threshold) + 1;
+      }
+      segs += n;
+      longs += n != 0;
+    }
+    // exclusive sums over the threads
+    before_longs = longs;
+    before_segs = segs;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t a = __shfl_up_sync(0xffffffffu, before_longs, o), b = __shfl_up_sync(0xffffffffu, before_segs, o);
+      if (lane >= o) {
+        before_longs += a;
+        before_segs += b;
+      }
+    }
+    if (lane == 31) {
+      scan[0][warp] = before_longs;
+      scan[1][warp] = before_segs;
+    }
+    __syncthreads();
+    before_longs -= longs;
+    before_segs -= segs;
+    all_longs = all_segs = 0;
+    for (int w = 0; w < kTableThreads / 32; ++w) {
+      if (w == warp) {
+        before_longs += all_longs;
+        before_segs += all_segs;
+      }
+      all_longs += scan[0][w];
+      all_segs += scan[1][w];
+    }
+    if (all_segs <= P.max_segments || threshold >= 1u << 30) break;
+    threshold *= 2;
+    __syncthreads();  // scan is read
+  }
+  if (all_segs > P.max_segments) {  // (a row of 2^30 entries: no plan holds one)
+    all_longs = all_segs = 0;
+    threshold = 0xffffffffu;
+  }
+  if (threadIdx.x == 0) {
+    P.table->threshold = threshold;
+    P.table->num_segments = all_segs;
+    P.table->num_long = all_longs;
+    P.long_first[all_longs] = all_segs;
+  }
+  if (threadIdx.x <= M.levels) {  // lower bound of the level's first node
+    const uint32_t node = M.level_node_offset[threadIdx.x];
+    uint32_t lo = 0, hi = M.num_domains;
+    while (lo < hi) {
+      const uint32_t mid = (lo + hi) / 2;
+      if (M.dom_node_ptr[mid] < node) lo = mid + 1;
+      else hi = mid;
+    }
+    P.table->level_domain[threadIdx.x] = lo;
+  }
+  if (all_longs == 0) return;
+  if (longs) {
+    for (uint32_t i = r0; i < r1; ++i) {
+      uint32_t n = 0;
+      for (int s = 0; s < P.nsets; ++s) {
+        const uint32_t len = P.sets[s].row_ptr[i + 1] - P.sets[s].row_ptr[i];
+        if (len > threshold) n += (len - 1) / (2 * threshold) + 1;
+      }
+      if (!n) continue;
+      P.long_row[before_longs] = i;
+      P.long_first[before_longs++] = before_segs;
+      before_segs += n;
+    }
+  }
+  __syncthreads();
+  for (uint32_t k = warp; k < all_longs; k += kTableThreads / 32) {  // a warp a row
+    const uint32_t i = P.long_row[k];
+    uint32_t at = P.long_first[k];
+    for (int s = 0; s < P.nsets; ++s) {
+      const uint32_t e0 = P.sets[s].row_ptr[i], e1 = P.sets[s].row_ptr[i + 1];
+      if (e1 - e0 <= threshold) continue;
+      const uint32_t n = (e1 - e0 - 1) / (2 * threshold) + 1;
+      for (uint32_t j = lane; j < n; j += 32) {
+        const uint32_t e = e0 + j * 2 * threshold;
+        P.segments[at + j] = make_uint4(i, e, min(e1, e + 2 * threshold), (uint32_t)s);
+      }
+      at += n;
+    }
   }
 }
 

@@ -463,7 +463,9 @@ uint64_t ys_pcg_workspace_doubles(uint32_t n) {
   // slots + partials + tickets
   // partials: up to 4 values per block of the row kernels, or 1 per block of
   // the kRowLanes-per-row SpMV (kRowLanes times more blocks)
-  return 4ull * 3 * nv + 2 * nv + ys::kSlots + (uint64_t)ys::kRowLanes * (grid + 2) + 8;
+  // and, for systems of its sizes, what the one-kernel MAS loop keeps
+  return 4ull * 3 * nv + 2 * nv + ys::kSlots + (uint64_t)ys::kRowLanes * (grid + 2) + 8 +
+         ys::mas_loop_workspace_doubles((uint32_t)nv);
 }
 
 int32_t ys_pcg_create(const ys_pcg_args* args, void** handle) {
@@ -555,7 +557,8 @@ int32_t ys_pcg_create(const ys_pcg_args* args, void** handle) {
     }
   }
   P.partials = w; w += (uint64_t)ys::kRowLanes * (grid + 2);
-  P.tickets = reinterpret_cast<unsigned*>(w);
+  P.tickets = reinterpret_cast<unsigned*>(w); w += 8;
+  h->mas.loop_workspace = w;
   P.jinv = a.jacobi_inverse;
   P.jgroup = a.jacobi_group;
   P.stop_rule = a.stop_rule;
@@ -605,7 +608,11 @@ int32_t ys_pcg_create(const ys_pcg_args* args, void** handle) {
       cudaGraphNode_t n1 = nullptr, n2 = nullptr, n3 = nullptr;
       void* args1[] = {&P};
       bool looped = false;
-      if (a.preconditioner == YS_PREC_MAS) e = ys::mas_add_loop_node(a.mas, body, &h->mas, &looped);
+      if (a.preconditioner == YS_PREC_MAS) {
+        cudaGraphNode_t tables = nullptr;
+        e = ys::mas_add_loop_node(a.mas, h->graph, body, &tables, &h->mas, &looped);
+        if (e == cudaSuccess && looped) e = cudaGraphAddDependencies(h->graph, &tables, &loop, 1);
+      }
       if (e != cudaSuccess || looped) {
         // one kernel runs every iteration
       } else if (streamed)
@@ -640,7 +647,6 @@ int32_t ys_pcg_create(const ys_pcg_args* args, void** handle) {
     if (h->exec) cudaGraphExecDestroy(h->exec);
     if (h->graph) cudaGraphDestroy(h->graph);
     if (h->slots_host) cudaFreeHost(h->slots_host);
-    if (h->mas.owned) cudaFree(h->mas.owned);
     delete h;
     return YS_ERR_CUDA;
   }
@@ -763,7 +769,6 @@ int32_t ys_pcg_destroy(void* handle) {
   if (h->exec) cudaGraphExecDestroy(h->exec);
   if (h->graph) cudaGraphDestroy(h->graph);
   if (h->slots_host) cudaFreeHost(h->slots_host);
-  if (h->mas.owned) cudaFree(h->mas.owned);
   delete h;
   return YS_OK;
 }

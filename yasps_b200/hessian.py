@@ -20,6 +20,7 @@ Pipeline (all on the device through libys_newton.so):
 
 from __future__ import annotations
 
+import itertools
 from typing import List, Optional
 
 import numpy as np
@@ -369,12 +370,17 @@ class _Term:
 
 
 class _Pattern:
-  """Device pattern + assembly plan of one occurrence set."""
+  """Device pattern + assembly plan of one occurrence set.  ``serial`` names
+  it for the caches of structure built on it: neither its address nor those
+  of its buffers would do, a later pattern may be given either."""
+
+  _serials = itertools.count()
 
   def __init__(self, coords, dims, m):
     import ctypes
     torch = _torch()
     self.m = m
+    self.serial = next(_Pattern._serials)
     cap = max(m, 1)
     i32 = lambda k: torch.empty(max(k, 1), dtype=torch.int32, device=_dev())
     self.positions = i32(2 * cap)

@@ -91,11 +91,12 @@ class _PcgBase:
   def _run_pcg(self, H, rhs, x, fp32, prec_kind, jinv, mas_handle, tol, maxit, zero_guess, stop_rule, jgroup=None):
     """One device PCG solve into ``x``; returns the ys_pcg_result."""
     # the graph holds every device pointer of the matrix: a rebuilt pattern
-    # (dynamic terms) gives new row plans and must give a new graph
+    # (dynamic terms) gives new row plans and must give a new graph, also
+    # where its buffers are those of the one before
     # (an FP32 solve first refreshes the streamed SpMV's packed blocks from
     # the current FP32 values; the graph holds the plan's pointers)
     streams = [H.stream_plan(bs) if fp32 and len(H.block_sets) == 1 else None for bs in H.block_sets]
-    plans = tuple(tuple(t.data_ptr() for t in H.spmv_plan(bs)) + (bs.pattern.num_unique,) +
+    plans = tuple(tuple(t.data_ptr() for t in H.spmv_plan(bs)) + (bs.pattern.serial, bs.pattern.num_unique) +
                   tuple(0 if t is None else (t.data_ptr() if hasattr(t, "data_ptr") else t) for t in H.tile_plan(bs)) +
                   (sp.pointers() if sp is not None else ())
                   for bs, sp in zip(H.block_sets, streams))
@@ -335,7 +336,7 @@ class masSolver(_PcgBase):
       raise NotImplementedError("the device MAS takes a static and at most one dynamic 3x3 block set")
     bs = sets[0]
     dyn = sets[1] if len(sets) == 2 else None
-    key = (id(bs.pattern), None if dyn is None else id(dyn.pattern), H.rows)
+    key = (bs.pattern.serial, None if dyn is None else dyn.pattern.serial, H.rows)
     if key == self._mas_key:
       return
     if self._mas is not None:
@@ -345,7 +346,7 @@ class masSolver(_PcgBase):
       raise NotImplementedError("the device MAS supports 3x3 blocks (3-DoF variables)")
     pos = bs.pattern.positions[:2 * bs.pattern.num_unique].cpu().numpy().astype(np.int64).reshape(-1, 2)
     nv = H.rows // 3
-    hkey = (id(bs.pattern), H.rows)
+    hkey = (bs.pattern.serial, H.rows)
     if getattr(self, "_hierarchy_key", None) != hkey or self.hierarchy is None:
       edges = pos[pos[:, 0] != pos[:, 1]] // 3
       self.hierarchy = mas_hierarchy.build_hierarchy(np.full(nv, 3), edges, self.max_domain_dofs, self.max_levels,
