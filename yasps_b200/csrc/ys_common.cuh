@@ -32,6 +32,22 @@ namespace ys {
 
 constexpr int kSMs = 148;  // B200: 2 dies x 74 SMs
 
+// Opens a kernel to as much dynamic shared memory as fits beside its static
+// shared memory; *most gets that.  The limit belongs to the function for the
+// whole process: set to what one launch needs, it would refuse the larger
+// launches of a handle that was made before.
+inline cudaError_t allow_dynamic_smem(const void* kernel, size_t* most = nullptr) {
+  int dev = 0, optin = 0;
+  cudaFuncAttributes fa{};
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, kernel);
+  if (e != cudaSuccess) return e;
+  const size_t room = (size_t)optin - fa.sharedSizeBytes;
+  if (most) *most = room;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room);
+}
+
 inline unsigned grid_for(uint64_t n, unsigned block) {
   uint64_t g = (n + block - 1) / block;
   return g == 0 ? 1u : (unsigned)(g > 0x7fffffffULL ? 0x7fffffffULL : g);

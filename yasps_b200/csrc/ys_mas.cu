@@ -897,19 +897,16 @@ constexpr uint32_t kLoopMaxVars = 110000;
 template <typename T, bool WIDE>
 static cudaError_t add_loop_kernel(cudaGraph_t body, cudaGraphNode_t* node, LoopParams& L, uint32_t nv, int sms,
                                    bool* used) {
-  int dev = 0, per_sm = 0, smem_max = 0;
+  int per_sm = 0;
+  size_t most = 0;
   const void* fn = (const void*)mas_pcg_loop<T, WIDE>;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  cudaFuncAttributes fa{};
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, fn);
+  cudaError_t e = allow_dynamic_smem(fn, &most);
   if (e != cudaSuccess) return e;
-  const size_t area = 16ull * L.area, room = (size_t)smem_max - fa.sharedSizeBytes - 1024;
-  L.gemv_warps = (uint32_t)std::min<size_t>(kLoopThreads / 32, room / area);
+  const size_t area = 16ull * L.area;
+  L.gemv_warps = (uint32_t)std::min<size_t>(kLoopThreads / 32, (most - 1024) / area);
   if (L.gemv_warps == 0) return cudaSuccess;
   const size_t smem = WIDE ? 2 * area : area * L.gemv_warps;  // the wide form: one area of doubles
-  e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kLoopThreads, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kLoopThreads, smem);
   if (e != cudaSuccess || per_sm < 1) return e;
   // 64 rows a pass of a CTA; the wide form a domain a CTA (tiny systems take
   // fewer CTAs: cheaper barriers)
@@ -1036,10 +1033,8 @@ int32_t ys_mas_create(const ys_mas_desc* d, void** handle) {
   M.fine_values = nullptr;
   cudaError_t e = cudaSuccess;
   {
-    const size_t smem = sizeof(double) * d->max_domain_dofs * d->max_domain_dofs;
-    e = cudaFuncSetAttribute(ys::mas_domain_inverse<6, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(ys::mas_domain_inverse<8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = ys::allow_dynamic_smem((const void*)ys::mas_domain_inverse<6, 4>);
+    if (e == cudaSuccess) e = ys::allow_dynamic_smem((const void*)ys::mas_domain_inverse<8, 4>);
     // prefer the largest shared-memory carveout so two 96-DoF domains fit per SM
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(ys::mas_domain_inverse<6, 4>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);

@@ -524,8 +524,6 @@ int32_t ys_pcg_create(const ys_pcg_args* args, void** handle) {
     tile_smem = ys::stream_smem_bytes(sp.block_cap, sp.entry_cap, sp.halo_cap, stages ? stages : 2);
     if (stages && cudaGetDevice(&dev) == cudaSuccess &&
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-        cudaFuncSetAttribute(ys::pcg_spmv_dot_streamed, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)tile_smem) == cudaSuccess &&
         sms > 0 && per_sm > 0) {
       const unsigned ntiles = (P.nv + ys::kTileRows - 1) / ys::kTileRows;
       grid_tiles = std::min<unsigned>(ntiles, (unsigned)(sms * per_sm));
@@ -543,8 +541,7 @@ int32_t ys_pcg_create(const ys_pcg_args* args, void** handle) {
     tile_smem = ys::tile_smem_bytes(a.matrix.tile_cap[0], a.matrix.entry_cap[0], stages);
     if (tile_smem <= 200u * 1024u &&
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-        cudaFuncSetAttribute(ys::pcg_spmv_dot_tiled, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem) ==
-            cudaSuccess &&
+        ys::allow_dynamic_smem((const void*)ys::pcg_spmv_dot_tiled) == cudaSuccess &&
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ys::pcg_spmv_dot_tiled, ys::kTileThreads, tile_smem) ==
             cudaSuccess &&
         sms > 0 && per_sm > 0) {

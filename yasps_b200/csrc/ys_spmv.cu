@@ -489,7 +489,7 @@ int32_t ys_spmv3_x32_tiled(const float* values32, const uint32_t* row_ptr, const
   if (stages == 0) stages = ys::tile_auto_stages(tile_cap, entry_cap, (size_t)smem_sm);
   const size_t smem = ys::tile_smem_bytes(tile_cap, entry_cap, stages);
   YS_REQUIRE(smem <= 200u * 1024u, YS_ERR_CAPACITY, "a tile's blocks exceed the shared-memory stage");
-  YS_CUDA_TRY(cudaFuncSetAttribute(ys::spmv3_x32_tiled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  YS_CUDA_TRY(ys::allow_dynamic_smem((const void*)ys::spmv3_x32_tiled_kernel));
   YS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ys::spmv3_x32_tiled_kernel, ys::kTileThreads,
                                                             smem));
   YS_REQUIRE(per_sm > 0, YS_ERR_CAPACITY, "tiled SpMV does not fit on an SM");
@@ -580,7 +580,7 @@ int32_t ys_spmv3_x32_streamed(const ys_spmv_stream* plan, const float* values32,
   YS_REQUIRE(stages != 0, YS_ERR_CAPACITY, "a tile's stream exceeds the shared-memory stages");
   const size_t smem = ys::stream_smem_bytes(plan->block_cap, plan->entry_cap, plan->halo_cap, stages);
   YS_REQUIRE(smem <= 220u * 1024u, YS_ERR_CAPACITY, "a tile's stream exceeds the shared-memory stages");
-  YS_CUDA_TRY(cudaFuncSetAttribute(ys::spmv3_x32_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  YS_CUDA_TRY(ys::allow_dynamic_smem((const void*)ys::spmv3_x32_stream_kernel));
   YS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ys::spmv3_x32_stream_kernel, ys::kTileThreads,
                                                             smem));
   YS_REQUIRE(per_sm > 0, YS_ERR_CAPACITY, "streamed SpMV does not fit on an SM");

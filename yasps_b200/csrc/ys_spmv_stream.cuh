@@ -92,11 +92,12 @@ inline uint32_t stream_pick_stages(const void* kernel, uint32_t block_cap, uint3
                                    int* per_sm) {
   int best = 0;
   uint32_t pick = 0;
+  *per_sm = 0;
+  if (allow_dynamic_smem(kernel) != cudaSuccess) return 0;
   for (uint32_t s = 3; s >= 2; --s) {
     const size_t smem = stream_smem_bytes(block_cap, entry_cap, halo_cap, s);
     int n = 0;
-    if (smem > 220u * 1024u || cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-                                   cudaSuccess ||
+    if (smem > 220u * 1024u ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kTileThreads, smem) != cudaSuccess)
       n = 0;
     if (n > best) {
