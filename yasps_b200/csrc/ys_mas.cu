@@ -398,6 +398,7 @@ struct MasPcg {
   int zero_guess;
   double tolerance;
   uint32_t max_it;
+  bool one_kernel;  // the loop is a body of a switch node (mas_pcg_loop)
   cudaGraphConditionalHandle cond;
 };
 
@@ -469,7 +470,10 @@ __global__ void __launch_bounds__(kPcgBlock) mas_init_collect(MasPcg P) {
   if (status == kContinue && P.st[kMaxItParam] < 1.0) status = kMaxIter;
   st[kTolAbs] = tol;
   st[kStatus] = (double)status;
-  cudaGraphSetConditional(P.cond, status == kContinue ? 1u : 0u);
+  if (P.one_kernel)  // a switch node: the body of that number, or none
+    cudaGraphSetConditional(P.cond, status == kContinue ? (unsigned)st[kBodyParam] : 0xffffffffu);
+  else
+    cudaGraphSetConditional(P.cond, status == kContinue ? 1u : 0u);
 }
 
 __global__ void __launch_bounds__(kPcgBlock) mas_update(MasPcg P) {
@@ -839,6 +843,7 @@ cudaError_t mas_add_init_nodes(void* mas, cudaGraph_t g, const cudaGraphNode_t* 
   P->tolerance = tolerance;
   P->max_it = max_it;
   P->cond = cond;
+  P->one_kernel = hooks->loop.used;
   h->pcgs.push_back(P);
   hooks->params = P;
   const unsigned grid = grid_for(nv, kPcgBlock);
@@ -894,33 +899,6 @@ cudaError_t mas_add_update_nodes(void* mas, cudaGraph_t body, const cudaGraphNod
 // the latency of data that comes from HBM.
 constexpr uint32_t kLoopMaxVars = 110000;
 
-template <typename T, bool WIDE>
-static cudaError_t add_loop_kernel(cudaGraph_t body, cudaGraphNode_t* node, LoopParams& L, uint32_t nv, int sms,
-                                   bool* used) {
-  int per_sm = 0;
-  size_t most = 0;
-  const void* fn = (const void*)mas_pcg_loop<T, WIDE>;
-  cudaError_t e = allow_dynamic_smem(fn, &most);
-  if (e != cudaSuccess) return e;
-  const size_t area = 16ull * L.area;
-  L.gemv_warps = (uint32_t)std::min<size_t>(kLoopThreads / 32, (most - 1024) / area);
-  if (L.gemv_warps == 0) return cudaSuccess;
-  const size_t smem = WIDE ? 2 * area : area * L.gemv_warps;  // the wide form: one area of doubles
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kLoopThreads, smem);
-  if (e != cudaSuccess || per_sm < 1) return e;
-  // 64 rows a pass of a CTA; the wide form a domain a CTA (tiny systems take
-  // fewer CTAs: cheaper barriers)
-  const unsigned want = std::max(grid_for(nv, kLoopThreads / 4), WIDE ? L.M.num_domains : 1u);
-  const unsigned grid = std::min<unsigned>(want, (unsigned)sms);
-  void* args[] = {&L};
-  e = add_kernel(body, node, nullptr, 0, fn, grid, kLoopThreads, smem, args);
-  cudaKernelNodeAttrValue cv{};
-  cv.cooperative = 1;
-  if (e == cudaSuccess) e = cudaGraphKernelNodeSetAttribute(*node, cudaKernelNodeAttributeCooperative, &cv);
-  *used = e == cudaSuccess;
-  return e;
-}
-
 // The loop's part of the solve's workspace (after 16-byte alignment).  The
 // partials take p.q, r.z and r.r of every CTA.  A system of at most
 // kLoopMaxGrid domains may run the wide form, whose FP64 corrections are one
@@ -952,14 +930,68 @@ static void loop_memory(LoopParams& L, uint32_t nv, double* w) {
   L.long_first = L.long_row + seg;
 }
 
-cudaError_t mas_add_loop_node(void* mas, cudaGraph_t g, cudaGraph_t body, cudaGraphNode_t* tables,
-                              MasPcgHooks* hooks, bool* used) {
-  *used = false;
-  auto* h = static_cast<MasHandle*>(mas);
-  auto* P = static_cast<MasPcg*>(hooks->params);
-  const MasDev& M = h->M;
-  if (P->nv > kLoopMaxVars) return cudaSuccess;
+// One solve takes every SM it has work for.  With one other in flight it takes
+// half of them and with more a quarter (a third would leave some CTAs four
+// virtual ones of 148 as well), so that they run side by side: a CTA fills its
+// SM's registers, and a grid that waits at barriers has to be resident as a
+// whole, so solves of a whole chip each run one after another.  Time a solve
+// with eight threads and streams, FP64 blocks, cubes of side 16 / 24 / 33 / 47:
+// 608 / 979 / 1650 / 4343 us on the whole chip each, 317 / 575 / 1421 / 3580
+// shared (the graph of kernels, slower alone: 248 / 447 / 1251 / 4370); in the
+// precision form 612 / 843 / 1440 / 3689, 341 / 502 / 1232 / 2847 shared (graph:
+// 315 / 494 / 1130 / 2989).
+cudaError_t mas_plan_loop(void* mas, int fp32, MasLoopPlan* loop) {
+  *loop = MasLoopPlan{};
+  const MasDev& M = static_cast<MasHandle*>(mas)->M;
+  if (M.nv > kLoopMaxVars) return cudaSuccess;
   if (M.levels > 2 && M.packed_nodes - M.level_node_offset[2] > kLoopCoarse) return cudaSuccess;
+  int dev = 0, sms = 0, coop = 0, per_sm = 0;
+  size_t most = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess || !coop) return e;
+  sms = std::min(sms, (int)kLoopMaxGrid);
+  loop->wide = M.num_domains <= (uint32_t)sms && M.packed_nodes <= loop_wide_nodes(M.nv);
+  static const void* const kernels[2][2][2] = {
+      {{(const void*)mas_pcg_loop<double, false, false>, (const void*)mas_pcg_loop<double, false, true>},
+       {(const void*)mas_pcg_loop<double, true, false>, (const void*)mas_pcg_loop<double, true, true>}},
+      {{(const void*)mas_pcg_loop<float, false, false>, (const void*)mas_pcg_loop<float, false, true>},
+       {(const void*)mas_pcg_loop<float, true, false>, (const void*)mas_pcg_loop<float, true, true>}}};
+  loop->kernel = kernels[fp32 ? 1 : 0][loop->wide ? 1 : 0][0];
+  loop->shared_kernel = kernels[fp32 ? 1 : 0][loop->wide ? 1 : 0][1];
+  size_t most_shared = 0;
+  e = allow_dynamic_smem(loop->kernel, &most);
+  if (e == cudaSuccess) e = allow_dynamic_smem(loop->shared_kernel, &most_shared);
+  if (e != cudaSuccess) return e;
+  most = std::min(most, most_shared);
+  const size_t area = gemv_smem_bytes(M.max_dofs);
+  loop->gemv_warps = (uint32_t)std::min<size_t>(kLoopThreads / 32, (most - 1024) / area);
+  if (loop->gemv_warps == 0) return cudaSuccess;
+  loop->smem = loop->wide ? 2 * area : area * loop->gemv_warps;  // the wide form: one area of doubles
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, loop->kernel, kLoopThreads, loop->smem);
+  if (e != cudaSuccess || per_sm < 1) return e;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, loop->shared_kernel, kLoopThreads, loop->smem);
+  if (e != cudaSuccess || per_sm < 1) return e;
+  // 64 rows a pass of a CTA; the wide form a domain a CTA (tiny systems take
+  // fewer CTAs: cheaper barriers)
+  const unsigned want = std::max(grid_for(M.nv, kLoopThreads / 4), loop->wide ? M.num_domains : 1u);
+  loop->blocks = std::min<unsigned>(want, (unsigned)sms);
+  for (int k = 0; k < kLoopShares; ++k) {
+    const int parts = k < 2 ? k + 1 : kLoopShares;
+    const unsigned grid = std::min<unsigned>(loop->blocks, (unsigned)((sms + parts - 1) / parts));
+    if (loop->bodies == 0 || grid != loop->grid[loop->bodies - 1]) loop->grid[loop->bodies++] = grid;
+    loop->body_of[k] = loop->bodies - 1;
+  }
+  loop->used = true;
+  return cudaSuccess;
+}
+
+cudaError_t mas_add_loop_nodes(void* mas, cudaGraph_t g, const cudaGraph_t* bodies, cudaGraphNode_t* tables,
+                               MasPcgHooks* hooks) {
+  const MasDev& M = static_cast<MasHandle*>(mas)->M;
+  auto* P = static_cast<MasPcg*>(hooks->params);
+  const MasLoopPlan& loop = hooks->loop;
   LoopParams L{};
   for (int s = 0; s < P->nsets; ++s) L.sets[s] = P->sets[s];
   L.nsets = P->nsets;
@@ -971,27 +1003,22 @@ cudaError_t mas_add_loop_node(void* mas, cudaGraph_t g, cudaGraph_t body, cudaGr
   L.q = P->q;
   L.st = P->st;
   L.arrivals = reinterpret_cast<unsigned long long*>(P->tickets + 4);
+  L.blocks = loop.blocks;
   L.stop_rule = P->stop_rule;
+  L.gemv_warps = loop.gemv_warps;
   L.area = (uint32_t)(gemv_smem_bytes(M.max_dofs) / 16);
-  L.cond = P->cond;
-  int dev = 0, sms = 0, coop = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e != cudaSuccess || !coop) return e;
-  sms = std::min(sms, (int)kLoopMaxGrid);
-  const bool wide = M.num_domains <= (uint32_t)sms && M.packed_nodes <= loop_wide_nodes(P->nv);
   loop_memory(L, P->nv, hooks->loop_workspace);
-  cudaGraphNode_t node = nullptr;
-  if (wide)
-    e = P->fp32 ? add_loop_kernel<float, true>(body, &node, L, P->nv, sms, used)
-                : add_loop_kernel<double, true>(body, &node, L, P->nv, sms, used);
-  else
-    e = P->fp32 ? add_loop_kernel<float, false>(body, &node, L, P->nv, sms, used)
-                : add_loop_kernel<double, false>(body, &node, L, P->nv, sms, used);
-  if (e != cudaSuccess || !*used) return e;
   void* args[] = {&L};
-  return add_kernel(g, tables, nullptr, 0, (const void*)loop_tables_kernel, 1, kTableThreads, 0, args);
+  cudaError_t e = add_kernel(g, tables, nullptr, 0, (const void*)loop_tables_kernel, 1, kTableThreads, 0, args);
+  for (int b = 0; b < loop.bodies && e == cudaSuccess; ++b) {
+    cudaGraphNode_t node = nullptr;
+    const void* kernel = loop.grid[b] == loop.blocks ? loop.kernel : loop.shared_kernel;
+    e = add_kernel(bodies[b], &node, nullptr, 0, kernel, loop.grid[b], kLoopThreads, loop.smem, args);
+    cudaKernelNodeAttrValue cv{};
+    cv.cooperative = 1;
+    if (e == cudaSuccess) e = cudaGraphKernelNodeSetAttribute(node, cudaKernelNodeAttributeCooperative, &cv);
+  }
+  return e;
 }
 
 }  // namespace ys

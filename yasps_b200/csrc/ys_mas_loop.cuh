@@ -1,5 +1,5 @@
 // The MAS-PCG iterations of a small or medium system in one cooperative
-// kernel (ys_mas.cu adds it as the body of the solve's conditional node).
+// kernel (ys_mas.cu adds it as a body of the solve's conditional node).
 //
 // A graph of five to seven kernels an iteration costs its launches and the
 // tails of grids that are far too small for the chip, where the data of an
@@ -30,10 +30,17 @@
 // that stands in the caller's buffers at each launch, as every other read of
 // the plan does.
 //
+// The sums are formed by P.blocks virtual CTAs, whatever number of CTAs runs
+// them (each takes every gridDim.x-th one).  A solve that has the chip to itself
+// runs them all at once; solves in flight on other streams share the chip, a
+// part of the SMs each (mas_plan_loop has the sizes), and since no sum
+// depends on the grid a solution has the same bits either way.
+//
 // Barrier waits are bounded (kPollLimitParam polls): a CTA that gives up marks
 // the solve void (kBarrierFail) and every CTA leaves.
 #pragma once
 
+#include "ys_mas.cuh"
 #include "ys_mas_dev.cuh"
 #include "ys_pcg.cuh"
 
@@ -65,6 +72,7 @@ struct LoopParams {
   double* st;
   double* partials;
   unsigned long long* arrivals;
+  uint32_t blocks;         // virtual CTAs: every sum is split among these
   int stop_rule;
   uint32_t gemv_warps;     // warps of a CTA with a GEMV area in shared memory
   uint32_t area;           // float4 of one area
@@ -77,7 +85,6 @@ struct LoopParams {
   uint32_t max_segments;   // room in segments, long_row and seg
   double* seg;             // 3 per segment
   double* zl64;            // the wide form's FP64 level corrections, 3 per packed node
-  cudaGraphConditionalHandle cond;
 };
 
 // Values other CTAs write in this kernel are read by plain loads (never the
@@ -147,19 +154,37 @@ __device__ __forceinline__ bool loop_barrier(const LoopParams& P, LoopState& S) 
 
 // Total of the grid's partials, by every warp for itself (all lanes get it, the
 // same bits in every warp and CTA): no CTA barrier on the path.
-__device__ __forceinline__ double loop_total(const double* partials) {
+__device__ __forceinline__ double loop_total(const double* partials, uint32_t blocks) {
   double a = 0.0;
-  for (unsigned b = threadIdx.x & 31; b < gridDim.x; b += 32) a += partials[b];
+  for (uint32_t b = threadIdx.x & 31; b < blocks; b += 32) a += partials[b];
   return warp_sum(a);
+}
+
+// A virtual CTA's sum, in two parts: every warp leaves its own in row k of
+// `parts` (k counts the CTA's virtual ones), and once all are there a warp a
+// virtual CTA adds the rows.  Nothing waits between the virtual CTAs.
+constexpr int kLoopWarps = kLoopThreads / 32;
+__device__ __forceinline__ void loop_part(double* parts, int k, double v) {
+  v = warp_sum(v);
+  if ((threadIdx.x & 31) == 0) parts[k * kLoopWarps + (threadIdx.x >> 5)] = v;
+}
+template <bool SHARED>
+__device__ __forceinline__ void loop_parts_end(uint32_t blocks, const double* parts, double* partials) {
+  const uint32_t lane = threadIdx.x & 31, k = threadIdx.x >> 5, vb = blockIdx.x + k * gridDim.x;
+  __syncthreads();
+  if (k < (SHARED ? kLoopShares : 1) && vb < blocks) {
+    const double t = warp_sum(lane < kLoopWarps ? parts[k * kLoopWarps + lane] : 0.0);
+    if (lane == 0) partials[vb] = t;
+  }
 }
 
 // The long rows' segments, a warp each; returns the lane's share of p.q.
 template <typename T>
 __device__ __forceinline__ double loop_segments(const LoopParams& P, const LoopState& L,
-                                                const typename LoopTypes<T>::X* px) {
+                                                const typename LoopTypes<T>::X* px, uint32_t vb, uint32_t blocks) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double dot = 0.0;
-  for (uint32_t s = warp * gridDim.x + blockIdx.x; s < L.t.num_segments; s += (kLoopThreads / 32) * gridDim.x) {
+  for (uint32_t s = warp * blocks + vb; s < L.t.num_segments; s += kLoopWarps * blocks) {
     const uint4 it = __ldg(P.segments + s);
     const SpmvSet& S = P.sets[it.w];
     const T* vals = set_values(S, T(0));
@@ -223,12 +248,12 @@ struct LoopRows {
 };
 
 // q = H p for this CTA's rows over one block set; returns the thread's share
-// of p.q.  R holds the first round's rows on entry and the first round's again
-// on exit.
+// of p.q.  R holds the first round's rows on entry and those from `next` on
+// exit.
 template <typename T, int U>
 __device__ __forceinline__ double loop_spmv(const LoopParams& P, const LoopState& L,
                                             const typename LoopTypes<T>::X* px, LoopRows<T, U>& R, uint32_t first,
-                                            uint32_t r1) {
+                                            uint32_t r1, uint32_t next, uint32_t next_r1) {
   constexpr uint32_t kRows = kLoopThreads / 8;
   const int sub = threadIdx.x & 7;
   const SpmvSet& S = P.sets[0];
@@ -261,9 +286,9 @@ __device__ __forceinline__ double loop_spmv(const LoopParams& P, const LoopState
 #pragma unroll
           for (int k = 0; k < 3; ++k) pr[u][k] = P.p[3ull * i + k];
       }
-      // the next round's rows (the first round's after the last)
+      // the next round's rows (those from `next` after the last)
       const bool more = wb + U * kRows < r1;
-      R.bounds(P, L, more ? base + U * kRows : first, r1);
+      R.bounds(P, L, more ? base + U * kRows : next, more ? r1 : next_r1);
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         a[u][0] = a[u][1] = a[u][2] = 0;
@@ -609,16 +634,18 @@ __device__ __forceinline__ void loop_collect(const LoopParams& P, uint32_t i, do
   }
 }
 
-template <typename T, bool WIDE>
+// SHARED: fewer CTAs than virtual ones (the other form is spared the loops over
+// them, and their registers: solve of a 33^3 cube in FP64 1702 -> 1655 us).
+template <typename T, bool WIDE, bool SHARED>
 __global__ void __launch_bounds__(kLoopThreads, 1) mas_pcg_loop(const __grid_constant__ LoopParams P) {
   extern __shared__ float4 loop_areas[];
-  __shared__ double red[kLoopThreads / 32];
+  __shared__ double parts[kLoopShares * kLoopWarps];
   __shared__ double coarse[3 * kLoopCoarse];
   __shared__ LoopState S;
   const MasDev& M = P.M;
   double* const st = P.st;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int kWarps = kLoopThreads / 32;
+  const uint32_t blocks = SHARED ? P.blocks : gridDim.x;
   const typename LoopTypes<T>::X* px;
   if constexpr (sizeof(T) == 4) px = P.p32;
   else px = P.p;
@@ -633,45 +660,64 @@ __global__ void __launch_bounds__(kLoopThreads, 1) mas_pcg_loop(const __grid_con
     S.t = *P.table;
   }
   __syncthreads();
-  // this CTA's rows
-  const uint32_t per = ((M.nv + gridDim.x - 1) / gridDim.x + 3u) & ~3u;
-  const uint32_t r1 = min(M.nv, (blockIdx.x + 1) * per);
-  const uint32_t first_row = blockIdx.x * per + (threadIdx.x >> 3);
+  // rows of a virtual CTA
+  const uint32_t per = ((M.nv + blocks - 1) / blocks + 3u) & ~3u;
+  auto rows_end = [&](uint32_t vb) { return min(M.nv, (vb + 1) * per); };
+  auto rows_begin = [&](uint32_t vb) { return vb * per + (threadIdx.x >> 3); };
   constexpr int U = 1;  // 2 spilled registers: slower
   LoopRows<T, U> rows;
   if (P.nsets == 1) {
-    rows.bounds(P, S, first_row, r1);
+    rows.bounds(P, S, rows_begin(blockIdx.x), rows_end(blockIdx.x));
     rows.indices(P, threadIdx.x & 7);
   }
   __syncthreads();
   while (S.status == kContinue) {
     // A
-    {
-      double dot = P.nsets == 1 ? loop_spmv<T, U>(P, S, px, rows, first_row, r1)
-                                : loop_spmv_sets<T>(P, S, px, first_row, r1);
-      if (S.t.num_segments) dot += loop_segments<T>(P, S, px);
-      const double s = block_sum<kLoopThreads>(dot, red);
-      if (threadIdx.x == 0) P.partials[blockIdx.x] = s;
+    int k = 0;  // counts the CTA's virtual ones
+    for (uint32_t vb = blockIdx.x; vb < blocks; vb += gridDim.x, ++k) {
+      const uint32_t first_row = rows_begin(vb), r1 = rows_end(vb);
+      double dot;
+      if (P.nsets == 1) {
+        // what the warp multiplies next: its rows of the CTA's next virtual
+        // CTA, or of the first one where that one has none for it
+        uint32_t nb = vb;
+        if constexpr (SHARED) nb += gridDim.x;
+        if (nb >= blocks || nb * per + 4u * warp >= M.nv) nb = blockIdx.x;
+        dot = loop_spmv<T, U>(P, S, px, rows, first_row, r1, rows_begin(nb), rows_end(nb));
+      } else {
+        dot = loop_spmv_sets<T>(P, S, px, first_row, r1);
+      }
+      if (S.t.num_segments) dot += loop_segments<T>(P, S, px, vb, blocks);
+      loop_part(parts, k, dot);
+      if constexpr (!SHARED) break;
     }
+    loop_parts_end<SHARED>(blocks, parts, P.partials);
     if (!loop_barrier(P, S)) break;
     // the first variables of B are on their way while the step length is summed
     LoopUpdate up;
     uint32_t up_i = 0, up_p = 0, up_q = 0, up_end = 0;
     bool up_on = false;
-    if (M.levels > 1) {
-      up_p = M.level_node_offset[1] + warp * gridDim.x + blockIdx.x;
-      if (up_p < M.level_node_offset[2]) {
-        up_end = __ldg(M.child_ptr + (up_p - M.nv) + 1);
-        up_q = __ldg(M.child_ptr + (up_p - M.nv)) + lane;
+    auto up_node = [&](uint32_t p) {  // the children of level-1 node p
+      up_p = p;
+      up_on = false;
+      if (p < M.level_node_offset[2]) {
+        up_end = __ldg(M.child_ptr + (p - M.nv) + 1);
+        up_q = __ldg(M.child_ptr + (p - M.nv)) + lane;
         up_on = up_q < up_end;
         if (up_on) up_i = __ldg(M.child_fine + up_q);
       }
-    } else {
-      up_i = blockIdx.x * kLoopThreads + threadIdx.x;
-      up_on = up_i < M.nv;
-    }
-    if (up_on) up.load(P, S, up_i);
-    const double curv = loop_total(P.partials), prev = S.delta;
+    };
+    auto up_first = [&](uint32_t vb) {
+      if (M.levels > 1) {
+        up_node(M.level_node_offset[1] + warp * blocks + vb);
+      } else {
+        up_i = vb * kLoopThreads + threadIdx.x;
+        up_on = up_i < M.nv;
+      }
+      if (up_on) up.load(P, S, up_i);
+    };
+    up_first(blockIdx.x);
+    const double curv = loop_total(P.partials, blocks), prev = S.delta;
     const bool restart = isfinite(curv) && curv <= 0.0 && isfinite(prev) && prev > 0.0;
     if (!restart && (!isfinite(curv) || curv <= 0.0)) {
       if (threadIdx.x == 0) {
@@ -686,10 +732,11 @@ __global__ void __launch_bounds__(kLoopThreads, 1) mas_pcg_loop(const __grid_con
     // (restart: finite non-positive curvature, zero step; see spmv_dot_finish)
     const double alpha = restart ? 0.0 : prev / curv;
     // B
-    double acc = 0.0;
-    {
+    k = 0;
+    for (uint32_t vb = blockIdx.x; vb < blocks; vb += gridDim.x, ++k) {
+      double acc = 0.0;
       if (M.levels > 1) {
-        for (; up_p < M.level_node_offset[2]; up_p += kWarps * gridDim.x) {  // warp-uniform
+        while (up_p < M.level_node_offset[2]) {  // warp-uniform
           double s[3] = {0.0, 0.0, 0.0};
           while (up_on) {
             acc += up.store(P, up_i, alpha);
@@ -705,30 +752,26 @@ __global__ void __launch_bounds__(kLoopThreads, 1) mas_pcg_loop(const __grid_con
 #pragma unroll
           for (int k = 0; k < 3; ++k) s[k] = warp_sum(s[k]);
           if (lane < 3) M.rl64[3ull * up_p + lane] = lane == 0 ? s[0] : (lane == 1 ? s[1] : s[2]);
-          const uint32_t np = up_p + kWarps * gridDim.x;
-          if (np < M.level_node_offset[2]) {
-            up_end = __ldg(M.child_ptr + (np - M.nv) + 1);
-            up_q = __ldg(M.child_ptr + (np - M.nv)) + lane;
-            up_on = up_q < up_end;
-            if (up_on) {
-              up_i = __ldg(M.child_fine + up_q);
-              up.load(P, S, up_i);
-            }
-          }
+          up_node(up_p + kLoopWarps * blocks);
+          if (up_on) up.load(P, S, up_i);
         }
       } else {
         while (up_on) {
           acc += up.store(P, up_i, alpha);
-          up_i += gridDim.x * kLoopThreads;
+          up_i += blocks * kLoopThreads;
           up_on = up_i < M.nv;
           if (up_on) up.load(P, S, up_i);
         }
       }
-      const double s = block_sum<kLoopThreads>(acc, red);
-      if (threadIdx.x == 0) P.partials[2 * gridDim.x + blockIdx.x] = s;
+      loop_part(parts, k, acc);
+      if constexpr (SHARED) {
+        if (vb + gridDim.x < blocks) up_first(vb + gridDim.x);
+      }
+      if constexpr (!SHARED) break;
     }
+    loop_parts_end<SHARED>(blocks, parts, P.partials + 2 * blocks);
     // the first tiles of the warp's (or CTA's) first domain are on their way
-    // over the barrier; the coarsest domains go to the first CTAs
+    // over the barrier; the coarsest domains go to the first virtual CTAs
     const uint32_t first2 = M.levels > 2 ? S.t.level_domain[2] : M.num_domains;
     const uint32_t first1 = M.levels > 1 ? S.t.level_domain[1] : M.num_domains, n1 = first2 - first1;
     const uint32_t whole = WIDE ? M.num_domains : M.num_domains - first2;  // domains by whole CTAs, from the last
@@ -741,24 +784,30 @@ __global__ void __launch_bounds__(kLoopThreads, 1) mas_pcg_loop(const __grid_con
     // The other CTAs share the rest, a warp a domain, when there are enough.
     const uint32_t n3 = !WIDE && M.levels > 3 ? M.num_domains - S.t.level_domain[3] : 0;
     const uint32_t n2 = WIDE ? 0 : whole - n3, nb2 = n2 > kLoopGroup ? (n2 + 2) / 3 : n2;
-    const uint32_t skip = !WIDE && n3 + nb2 < gridDim.x / 2 ? n3 + nb2 : 0;
-    const uint32_t whole_end = skip && blockIdx.x >= skip ? 0 : whole;
-    const uint32_t whole_step = !skip ? gridDim.x : (blockIdx.x < n3 ? whole : nb2);
-    const uint32_t workers = gridDim.x - skip;
-    uint32_t job = first2;
-    if (!WIDE && warp < (int)P.gemv_warps && blockIdx.x >= skip) job = warp * workers + (blockIdx.x - skip);
+    const uint32_t skip = !WIDE && n3 + nb2 < blocks / 2 ? n3 + nb2 : 0;
+    const uint32_t workers = blocks - skip;
+    auto whole_end = [&](uint32_t vb) { return skip && vb >= skip ? 0 : whole; };
+    auto first_job = [&](uint32_t vb) {
+      return !WIDE && warp < (int)P.gemv_warps && vb >= skip ? warp * workers + (vb - skip) : first2;
+    };
     LoopTilesAhead ahead;
-    if (blockIdx.x < whole_end) loop_prefetch(M, M.num_domains - 1 - blockIdx.x, ahead.t[0]);
-    else if (job < first2) ahead.first(M, job < n1 ? first1 + job : job - n1);
+    {
+      const uint32_t job = first_job(blockIdx.x);
+      if (blockIdx.x < whole_end(blockIdx.x)) loop_prefetch(M, M.num_domains - 1 - blockIdx.x, ahead.t[0]);
+      else if (job < first2) ahead.first(M, job < n1 ? first1 + job : job - n1);
+    }
     if (!loop_barrier(P, S)) break;
     // C
-    acc = 0.0;
-    {
-      for (uint32_t k = blockIdx.x; k < whole_end; k += whole_step) {
-        const uint32_t d = M.num_domains - 1 - k;
+    k = 0;
+    for (uint32_t vb = blockIdx.x; vb < blocks; vb += gridDim.x, ++k) {
+      double acc = 0.0;
+      // `ahead` holds the first tiles of the CTA's first virtual CTA
+      const uint32_t end = whole_end(vb), step = !skip ? blocks : (vb < n3 ? whole : nb2);
+      for (uint32_t w = vb; w < end; w += step) {
+        const uint32_t d = M.num_domains - 1 - w;
         uint32_t l = 0;
         while (l + 1 < M.levels && d >= S.t.level_domain[l + 1]) ++l;
-        if (k != blockIdx.x) loop_prefetch(M, d, ahead.t[0]);
+        if (w != blockIdx.x) loop_prefetch(M, d, ahead.t[0]);
         if (l >= 2) loop_coarse(P, d, l, coarse);
         const double* res = l >= 2 ? coarse : (l == 1 ? M.rl64 : P.r);
         const uint32_t base = l >= 2 ? M.level_node_offset[2] : 0u;
@@ -769,7 +818,8 @@ __global__ void __launch_bounds__(kLoopThreads, 1) mas_pcg_loop(const __grid_con
       }
       if constexpr (!WIDE) {
         float4* const area = loop_areas + (size_t)warp * P.area;
-        const bool fresh = blockIdx.x >= whole_end;  // `ahead` still holds the first job's tiles
+        const uint32_t job = first_job(vb);
+        const bool fresh = vb == blockIdx.x && vb >= end;  // `ahead` still holds the first job's tiles
         for (uint32_t j = job; j < first2; j += P.gemv_warps * workers) {
           const bool one = j < n1;  // the level-1 domains first
           const uint32_t d = one ? first1 + j : j - n1;
@@ -777,9 +827,10 @@ __global__ void __launch_bounds__(kLoopThreads, 1) mas_pcg_loop(const __grid_con
           acc += loop_gemv(P, d, ahead, one ? M.rl64 : P.r, 0u, (double)M.weight[one ? 1 : 0], area);
         }
       }
-      const double s = block_sum<kLoopThreads>(acc, red);
-      if (threadIdx.x == 0) P.partials[gridDim.x + blockIdx.x] = s;
+      loop_part(parts, k, acc);
+      if constexpr (!SHARED) break;
     }
+    loop_parts_end<SHARED>(blocks, parts, P.partials + blocks);
     if (!loop_barrier(P, S)) break;
     // the first z of D while the totals are summed
     double z[3] = {0.0, 0.0, 0.0}, pold[3] = {0.0, 0.0, 0.0};
@@ -789,7 +840,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) mas_pcg_loop(const __grid_con
 #pragma unroll
       for (int k = 0; k < 3; ++k) pold[k] = P.p[3ull * d_i + k];
     }
-    const double delta = loop_total(P.partials + gridDim.x), rr = loop_total(P.partials + 2 * gridDim.x);
+    const double delta = loop_total(P.partials + blocks, blocks), rr = loop_total(P.partials + 2 * blocks, blocks);
     double beta = 0.0;
     int status = kContinue;
     const double it = S.it + 1.0;
@@ -843,7 +894,6 @@ __global__ void __launch_bounds__(kLoopThreads, 1) mas_pcg_loop(const __grid_con
     st[kRR] = S.rr;
     st[kIter] = S.it;
     st[kStatus] = (double)S.status;
-    cudaGraphSetConditional(P.cond, 0u);
   }
 }
 

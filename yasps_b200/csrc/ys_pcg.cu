@@ -12,6 +12,8 @@
 // and a single device->host read of the status per solve.  All reductions are
 // deterministic (fixed-order block trees, fixed-order partial sums).
 #include <algorithm>
+#include <atomic>
+#include <chrono>
 #include <cmath>
 #include <vector>
 
@@ -438,7 +440,45 @@ struct PcgHandle {
   // tolerance, iteration budget, grid-barrier poll limit (copied to the
   // device per launch)
   double params[3] = {0.0, 0.0, (double)kDefaultPollLimit};
+  int device = 0;
+  bool in_flight = false;  // counted in g_flight
 };
+
+// One-kernel MAS solves launched and not yet waited for, a count a device, and
+// the times up to which two, three and four of them share the chip.  They only
+// choose how many SMs the next launch takes (mas_plan_loop): results do not
+// depend on them.  A count is kept for a few milliseconds, since a thread that
+// steps a scene is between two solves about half the time: on the whole chip
+// such a solve would hold the others up (four threads, precision form, cube of
+// side 16 / 33 / 47: 436 -> 406, 1390 -> 1330, 3025 -> 2878 us a solve).
+constexpr int kMaxDevices = 64;
+constexpr std::chrono::milliseconds kShareKept(5);
+struct Flight {
+  std::atomic<int> count{0};
+  std::atomic<int64_t> until[kLoopShares] = {};
+};
+static Flight g_flight[kMaxDevices];
+
+// Counts the solve in; returns how many share the chip.
+static int enter_flight(PcgHandle* h) {
+  Flight& f = g_flight[h->device % kMaxDevices];
+  const int n = h->in_flight ? f.count.load() : f.count.fetch_add(1) + 1;
+  h->in_flight = true;
+  const auto now = std::chrono::steady_clock::now().time_since_epoch();
+  const int64_t t = std::chrono::duration_cast<std::chrono::nanoseconds>(now).count();
+  const int64_t kept = t + std::chrono::duration_cast<std::chrono::nanoseconds>(kShareKept).count();
+  int share = 1;
+  for (int k = 2; k <= kLoopShares; ++k) {
+    if (n >= k) f.until[k - 1].store(kept);
+    if (f.until[k - 1].load() > t) share = k;
+  }
+  return share;
+}
+
+static void leave_flight(PcgHandle* h) {
+  if (h->in_flight) g_flight[h->device % kMaxDevices].count.fetch_sub(1);
+  h->in_flight = false;
+}
 
 static cudaError_t add_kernel(cudaGraph_t g, cudaGraphNode_t* node, const cudaGraphNode_t* deps, size_t ndeps,
                               const void* fn, unsigned grid, unsigned block, void** args, size_t smem = 0) {
@@ -567,7 +607,10 @@ int32_t ys_pcg_create(const ys_pcg_args* args, void** handle) {
   h->params[1] = (double)a.max_iterations;
   h->preconditioner = a.preconditioner;
 
-  cudaError_t e = cudaGraphCreate(&h->graph, 0);
+  cudaError_t e = cudaGetDevice(&h->device);
+  if (e == cudaSuccess && a.preconditioner == YS_PREC_MAS) e = ys::mas_plan_loop(a.mas, P.fp32, &h->mas.loop);
+  const ys::MasLoopPlan& one = h->mas.loop;
+  if (e == cudaSuccess) e = cudaGraphCreate(&h->graph, 0);
   if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&P.cond, h->graph, 0, cudaGraphCondAssignDefault);
   if (e == cudaSuccess) e = cudaMallocHost(&h->slots_host, sizeof(double) * ys::kSlots);
   cudaGraphNode_t reset = nullptr, init = nullptr, loop = nullptr;
@@ -597,21 +640,18 @@ int32_t ys_pcg_create(const ys_pcg_args* args, void** handle) {
     cudaGraphNodeParams cp{};
     cp.type = cudaGraphNodeTypeConditional;
     cp.conditional.handle = P.cond;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
+    // the one-kernel loop: a body for each grid it may run on
+    cp.conditional.type = one.used ? cudaGraphCondTypeSwitch : cudaGraphCondTypeWhile;
+    cp.conditional.size = one.used ? (unsigned)one.bodies : 1u;
     e = cudaGraphAddNode(&loop, h->graph, &init, 1, &cp);
     if (e == cudaSuccess) {
       cudaGraph_t body = cp.conditional.phGraph_out[0];
       cudaGraphNode_t n1 = nullptr, n2 = nullptr, n3 = nullptr;
       void* args1[] = {&P};
-      bool looped = false;
-      if (a.preconditioner == YS_PREC_MAS) {
+      if (one.used) {  // one kernel runs every iteration
         cudaGraphNode_t tables = nullptr;
-        e = ys::mas_add_loop_node(a.mas, h->graph, body, &tables, &h->mas, &looped);
-        if (e == cudaSuccess && looped) e = cudaGraphAddDependencies(h->graph, &tables, &loop, 1);
-      }
-      if (e != cudaSuccess || looped) {
-        // one kernel runs every iteration
+        e = ys::mas_add_loop_nodes(a.mas, h->graph, cp.conditional.phGraph_out, &tables, &h->mas);
+        if (e == cudaSuccess) e = cudaGraphAddDependencies(h->graph, &tables, &loop, 1);
       } else if (streamed)
         e = ys::add_kernel(body, &n1, nullptr, 0, (const void*)ys::pcg_spmv_dot_streamed, grid_tiles,
                            ys::kTileThreads, args1, tile_smem);
@@ -622,7 +662,7 @@ int32_t ys_pcg_create(const ys_pcg_args* args, void** handle) {
         e = ys::add_kernel(body, &n1, nullptr, 0,
                            P.fp32 ? (const void*)ys::pcg_spmv_dot<true> : (const void*)ys::pcg_spmv_dot<false>,
                            grid_rows, ys::kPcgBlock, args1);
-      if (e == cudaSuccess && !looped) {
+      if (e == cudaSuccess && !one.used) {
         if (a.preconditioner == YS_PREC_BLOCK_JACOBI) {
           e = ys::add_kernel(body, &n2, &n1, 1,
                              P.jgroup ? (const void*)ys::pcg_update_bjw : (const void*)ys::pcg_update_bj, grid,
@@ -631,7 +671,7 @@ int32_t ys_pcg_create(const ys_pcg_args* args, void** handle) {
           e = ys::mas_add_update_nodes(a.mas, body, &n1, 1, &n2, &h->mas);
         }
       }
-      if (looped || (e == cudaSuccess && a.preconditioner != YS_PREC_BLOCK_JACOBI && h->mas.fused_direction))
+      if (one.used || (e == cudaSuccess && a.preconditioner != YS_PREC_BLOCK_JACOBI && h->mas.fused_direction))
         n3 = n2;  // the MAS collect kernel updated p already
       else if (e == cudaSuccess)
         e = ys::add_kernel(body, &n3, &n2, 1, (const void*)ys::pcg_direction, grid, ys::kPcgBlock, args1);
@@ -656,10 +696,15 @@ int32_t ys_pcg_launch(void* handle, void* stream) {
   auto* h = static_cast<ys::PcgHandle*>(handle);
   // Pageable source: the copy is staged before the call returns, so the
   // parameters may change for the next launch right away.
-  const double params[3] = {h->params[0], h->params[1], h->params[2]};
-  YS_CUDA_TRY(cudaMemcpyAsync(h->P.st + ys::kTolParam, params, sizeof(params), cudaMemcpyHostToDevice,
-                              (cudaStream_t)stream));
-  YS_CUDA_TRY(cudaGraphLaunch(h->exec, (cudaStream_t)stream));
+  const ys::MasLoopPlan& one = h->mas.loop;
+  int body = 0;
+  if (one.used) body = one.body_of[ys::enter_flight(h) - 1];
+  const double params[4] = {h->params[0], h->params[1], h->params[2], (double)body};
+  cudaError_t e = cudaMemcpyAsync(h->P.st + ys::kTolParam, params, sizeof(params), cudaMemcpyHostToDevice,
+                                  (cudaStream_t)stream);
+  if (e == cudaSuccess) e = cudaGraphLaunch(h->exec, (cudaStream_t)stream);
+  if (e != cudaSuccess) ys::leave_flight(h);
+  YS_CUDA_TRY(e);
   return YS_OK;
 }
 
@@ -681,8 +726,10 @@ int32_t ys_pcg_status(void* handle, void* stream, ys_pcg_result* result) {
   YS_REQUIRE(handle && result, YS_ERR_INVALID, "null argument");
   auto* h = static_cast<ys::PcgHandle*>(handle);
   cudaStream_t s = (cudaStream_t)stream;
-  YS_CUDA_TRY(cudaMemcpyAsync(h->slots_host, h->P.st, sizeof(double) * ys::kSlots, cudaMemcpyDeviceToHost, s));
-  YS_CUDA_TRY(cudaStreamSynchronize(s));
+  cudaError_t e = cudaMemcpyAsync(h->slots_host, h->P.st, sizeof(double) * ys::kSlots, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  ys::leave_flight(h);
+  YS_CUDA_TRY(e);
   const double* st = h->slots_host;
   const int status = (int)st[ys::kStatus];
   const uint32_t it = (uint32_t)st[ys::kIter];
@@ -763,6 +810,7 @@ int32_t ys_refine_residual(const ys_matrix3* m, const double* rhs, double* x, co
 int32_t ys_pcg_destroy(void* handle) {
   if (!handle) return YS_OK;
   auto* h = static_cast<ys::PcgHandle*>(handle);
+  ys::leave_flight(h);
   if (h->exec) cudaGraphExecDestroy(h->exec);
   if (h->graph) cudaGraphDestroy(h->graph);
   if (h->slots_host) cudaFreeHost(h->slots_host);

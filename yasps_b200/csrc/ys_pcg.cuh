@@ -24,7 +24,8 @@ enum PcgSlot : int {
   kTolParam = 13,  // solve parameters, written by the host before each launch
   kMaxItParam = 14,
   kPollLimitParam = 15,  // polls a block makes at a grid barrier before it gives up
-  kRestart = 16,   // nonzero: this iteration took a zero step (non-positive curvature), beta = 0 next
+  kBodyParam = 16,  // body of the switch node that runs the one-kernel MAS loop
+  kRestart = 17,   // nonzero: this iteration took a zero step (non-positive curvature), beta = 0 next
   kSlots = 20
 };
 
