@@ -850,6 +850,10 @@ int32_t ys_pcg_status(void* handle, void* stream, ys_pcg_result* result);
  * (PKG/kernel/Solver/solverKernel.pyx:547-687, block-Jacobi) and the MAS
  * PCG runtime (PKG/solver/mas/cuda_runtime.py:3549-3751, mas/cuda/pcg.cu). */
 int32_t ys_pcg_create(const ys_pcg_args* args, void** handle);
+/* The same with the MAS loop always as a graph of kernels an iteration, the
+ * form of systems beyond the one-kernel loop's sizes.  The two forms sum in
+ * other orders, so their iteration counts and last digits differ.           */
+int32_t ys_pcg_create_kernels(const ys_pcg_args* args, void** handle);
 int32_t ys_pcg_run(void* handle, void* stream, ys_pcg_result* result);
 int32_t ys_pcg_destroy(void* handle);
 

@@ -10,6 +10,9 @@
 * The grid barrier of the MAS loop gives up after a host-set number of polls:
   a limit of zero makes every waiting block give up at once, the solve is
   reported void (YS_ERR_CUDA) and the context stays usable.
+
+Both for the one-kernel loop, which solves of these sizes take, and for the
+graph of kernels that larger ones run.
 """
 
 import numpy as np
@@ -24,7 +27,8 @@ from yasps_b200 import scenes
 pytestmark = pytest.mark.gpu
 
 
-def test_mas_restarts_on_non_positive_curvature():
+@pytest.mark.parametrize("one_kernel", [True, False])
+def test_mas_restarts_on_non_positive_curvature(one_kernel):
   import torch
   cube = scenes.fem_cube(8, spacing=0.1, young=1e5, poisson=0.4, noise=0.01, seed=3)
   ora = OracleCube(cube)
@@ -32,6 +36,7 @@ def test_mas_restarts_on_non_positive_curvature():
   sc.minimizer.setSolver("mas", max_levels=1, global_coarse_domain=False)
   H = sc.minimizer.computeNumericValue()
   impl = sc.minimizer.linearSolver.implementation
+  impl.one_kernel_loop = one_kernel
   impl._ensure_hierarchy(H)
   assert len(impl.hierarchy.levels) == 1 and len(impl.hierarchy.levels[0].domains) > 1
   p = ora.pattern
@@ -88,13 +93,15 @@ def pattern_matvec(p, vals, x):
   return pattern.spmv(p, vals, x)
 
 
-def test_mas_grid_barrier_poll_limit_voids_the_solve():
+@pytest.mark.parametrize("one_kernel", [True, False])
+def test_mas_grid_barrier_poll_limit_voids_the_solve(one_kernel):
   cube = scenes.fem_cube(10, spacing=0.1, young=1e5, poisson=0.4, noise=0.01, seed=0)
   ora = OracleCube(cube)
   sc, _ = scenes.fem_scene(cube)
   sc.minimizer.setSolver("mas")
   H = sc.minimizer.computeNumericValue()
   solver = sc.minimizer.linearSolver
+  solver.implementation.one_kernel_loop = one_kernel
   solve = lambda: solver.computeSolution(H, H.gradient, None, tolerance=1e-12, maxIterations=40,
                                          zero_initial_guess=True)
   assert solve() == 0

@@ -179,6 +179,7 @@ SIGNATURES = {
     "ys_spmv_stream_fill": (i32, [vp, vp, u64, vp, vp]),
     "ys_spmv3_x32_streamed": (i32, [P(SpmvStream), vp, vp, vp, vp, u32, vp, vp, i32, u32, u32, vp, vp]),
     "ys_pcg_workspace_doubles": (u64, [u32]),
+    "ys_pcg_create_kernels": (i32, [P(PcgArgs), P(vp)]),
     "ys_pcg_create": (i32, [P(PcgArgs), P(vp)]),
     "ys_pcg_run": (i32, [vp, vp, P(PcgResult)]),
     "ys_pcg_launch": (i32, [vp, vp]),

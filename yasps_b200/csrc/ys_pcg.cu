@@ -508,7 +508,7 @@ uint64_t ys_pcg_workspace_doubles(uint32_t n) {
          ys::mas_loop_workspace_doubles((uint32_t)nv);
 }
 
-int32_t ys_pcg_create(const ys_pcg_args* args, void** handle) {
+static int32_t pcg_create(const ys_pcg_args* args, bool one_kernel, void** handle) {
   YS_REQUIRE(args && handle, YS_ERR_INVALID, "null argument");
   const ys_pcg_args& a = *args;
   YS_REQUIRE(a.matrix.num_sets >= 1 && a.matrix.num_sets <= 2, YS_ERR_INVALID, "1 or 2 block sets");
@@ -608,7 +608,8 @@ int32_t ys_pcg_create(const ys_pcg_args* args, void** handle) {
   h->preconditioner = a.preconditioner;
 
   cudaError_t e = cudaGetDevice(&h->device);
-  if (e == cudaSuccess && a.preconditioner == YS_PREC_MAS) e = ys::mas_plan_loop(a.mas, P.fp32, &h->mas.loop);
+  if (e == cudaSuccess && one_kernel && a.preconditioner == YS_PREC_MAS)
+    e = ys::mas_plan_loop(a.mas, P.fp32, &h->mas.loop);
   const ys::MasLoopPlan& one = h->mas.loop;
   if (e == cudaSuccess) e = cudaGraphCreate(&h->graph, 0);
   if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&P.cond, h->graph, 0, cudaGraphCondAssignDefault);
@@ -690,6 +691,10 @@ int32_t ys_pcg_create(const ys_pcg_args* args, void** handle) {
   *handle = h;
   return YS_OK;
 }
+
+int32_t ys_pcg_create(const ys_pcg_args* args, void** handle) { return pcg_create(args, true, handle); }
+
+int32_t ys_pcg_create_kernels(const ys_pcg_args* args, void** handle) { return pcg_create(args, false, handle); }
 
 int32_t ys_pcg_launch(void* handle, void* stream) {
   YS_REQUIRE(handle, YS_ERR_INVALID, "null handle");

@@ -57,6 +57,10 @@ def _as_tensor(v):
 
 
 class _PcgBase:
+  # False: MAS solves of every size run the graph of kernels that those
+  # beyond the one-kernel loop's sizes run (ys_pcg_create_kernels)
+  one_kernel_loop = True
+
   def __init__(self, stop_rule="preconditioned"):
     if stop_rule not in _STOP:
       raise ValueError("stop_rule must be 'preconditioned' or 'residual'")
@@ -101,7 +105,7 @@ class _PcgBase:
                   (sp.pointers() if sp is not None else ())
                   for bs, sp in zip(H.block_sets, streams))
     key = (id(H), H.rows, rhs.data_ptr(), x.data_ptr(), fp32, prec_kind, None if jinv is None else jinv.data_ptr(),
-           mas_handle, bool(zero_guess), stop_rule, None if jgroup is None else jgroup.data_ptr(),
+           mas_handle, self.one_kernel_loop, bool(zero_guess), stop_rule, None if jgroup is None else jgroup.data_ptr(),
            tuple(bs.values.data_ptr() for bs in H.block_sets),
            tuple(0 if bs.values32 is None else bs.values32.data_ptr() for bs in H.block_sets), plans)
 
@@ -121,7 +125,8 @@ class _PcgBase:
       args.workspace = L.ptr(self._work)
       args.jacobi_group = L.ptr(jgroup)
       h = ctypes.c_void_p()
-      L.call("ys_pcg_create", ctypes.byref(args), ctypes.byref(h))
+      L.call("ys_pcg_create" if self.one_kernel_loop else "ys_pcg_create_kernels", ctypes.byref(args),
+             ctypes.byref(h))
       return h, args
 
     handle = self._cache.get(key, build)
