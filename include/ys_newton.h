@@ -831,16 +831,20 @@ int32_t ys_refine_residual(const ys_matrix3* m, const double* rhs, double* x, co
 /* Change the tolerance / iteration budget of an existing solver (the graph
  * reads them from device memory, so no rebuild). */
 int32_t ys_pcg_set_params(void* handle, double tolerance, uint32_t max_iterations);
-/* Polls a block of the MAS loop makes at its grid barrier (the cooperative
- * collect + direction kernel) before it gives up; default 2^24.  A block that
- * gives up marks the solve void and ys_pcg_status returns YS_ERR_CUDA; the
- * loop then ends at its iteration budget.  The waiting grid is co-resident,
- * so the default bound is never reached in a healthy run; a small bound
- * exercises the failure path without hanging the device.  Applies from the
- * next launch.  No counterpart in the reference (its loop has no grid-wide
+/* Polls a block of the MAS loop makes at a grid barrier (of the one-kernel
+ * loop, or of the cooperative collect + direction kernel of larger systems)
+ * before it gives up; default 2^24.  A block that gives up marks the solve
+ * void and ys_pcg_status returns YS_ERR_CUDA; the one-kernel loop ends there,
+ * the loop of kernels at its iteration budget.  The waiting grid is
+ * co-resident, so the default bound is never reached in a healthy run; a small
+ * bound exercises the failure path without hanging the device.  Applies from
+ * the next launch.  No counterpart in the reference (its loop has no grid-wide
  * wait).                                                                    */
 int32_t ys_pcg_set_barrier_poll_limit(void* handle, uint32_t polls);
-/* Asynchronous halves of ys_pcg_run. */
+/* Asynchronous halves of ys_pcg_run.  MAS solves of small and medium systems
+ * run their iterations in one cooperative kernel, on the whole chip when no
+ * other such solve of the process has been launched and not yet waited for
+ * (ys_pcg_status), else on a part of it; the solution does not depend on that. */
 int32_t ys_pcg_launch(void* handle, void* stream);
 int32_t ys_pcg_status(void* handle, void* stream, ys_pcg_result* result);
 
@@ -848,7 +852,13 @@ int32_t ys_pcg_status(void* handle, void* stream, ys_pcg_result* result);
  * on the device behind a conditional while node; one device->host read of
  * the status per solve).  Replaces `computeSolution`
  * (PKG/kernel/Solver/solverKernel.pyx:547-687, block-Jacobi) and the MAS
- * PCG runtime (PKG/solver/mas/cuda_runtime.py:3549-3751, mas/cuda/pcg.cu). */
+ * PCG runtime (PKG/solver/mas/cuda_runtime.py:3549-3751, mas/cuda/pcg.cu).
+ * The handle keeps the pointers of `args`: every launch reads the row plan,
+ * the blocks and the right-hand side that stand there at that point of its
+ * stream, so a plan that is rewritten in place (the same capacities) is
+ * followed.  What was derived from a plan is the caller's to renew with it:
+ * a tile or stream plan, and the tables of a MAS handle (a preconditioner of
+ * the old pattern slows a solve down, it does not change its answer).       */
 int32_t ys_pcg_create(const ys_pcg_args* args, void** handle);
 /* The same with the MAS loop always as a graph of kernels an iteration, the
  * form of systems beyond the one-kernel loop's sizes.  The two forms sum in
