@@ -893,10 +893,15 @@ cudaError_t mas_add_update_nodes(void* mas, cudaGraph_t body, const cudaGraphNod
   return e;
 }
 
-// Variables up to which the loop runs as one kernel (mas_pcg_loop): 24 us an
-// iteration against 34 for the graph of kernels at 31,744 variables (FEM cube,
-// FP32), 58 against 64 at 108,288, where the sixteen warps an SM no longer hide
-// the latency of data that comes from HBM.
+// Variables up to which the loop runs as one kernel (mas_pcg_loop).  Loop /
+// graph of kernels, us an iteration: FP32 cubes 24.6 / 35.9 at 34,848 variables,
+// 58.3 / 67.7 at 108,288, 72.3 / 75.6 at 137,904, 84.4 / 88.6 at 172,480, 106.7 /
+// 99.3 at 212,400; FP64 29.3 / 38.8, 71.8 / 78.6, 89.5 / 90.1, 105.4 / 107.3, 132.7 /
+// 123.5; cloth with bodies 58.2 / 71.5 (FP64 67.7 / 79.4) at 108,964, 68.1 / 76.0
+// (80.0 / 84.0) at 129,664.  The sixteen warps an SM do not hide the latency of
+// data that comes from HBM.  The line lies below the crossing (about 180,000):
+// past it the loop gives a few percent to a solve by itself, and kernels share
+// the chip better where several run.
 constexpr uint32_t kLoopMaxVars = 110000;
 
 // The loop's part of the solve's workspace (after 16-byte alignment).  The

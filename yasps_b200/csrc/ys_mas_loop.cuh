@@ -776,11 +776,12 @@ __global__ void __launch_bounds__(kLoopThreads, 1) mas_pcg_loop(const __grid_con
     const uint32_t first1 = M.levels > 1 ? S.t.level_domain[1] : M.num_domains, n1 = first2 - first1;
     const uint32_t whole = WIDE ? M.num_domains : M.num_domains - first2;  // domains by whole CTAs, from the last
     // of those, a CTA takes one of the levels >= 3 (their residuals are a chain
-    // of sums) and one of level 2, or three of many: 18 level-2 domains then
-    // leave 12 CTAs more to the fine levels (65,600 variables, cloth with
-    // bodies: 15.7 -> 14.0 ms a step in FP32, 16.4 -> 15.0 in FP64), where the
-    // few of a cube would only wait for one another.  The line at 12 lies
-    // between the two kinds, not at a measured crossing.
+    // of sums) and one of level 2, or three of many, which leaves more CTAs to
+    // the fine levels where a few would only wait for one another.  Apart /
+    // three to a CTA, us an iteration in FP32 (FP64) on cloths with bodies:
+    // 26.1 / 27.5 (30.4 / 31.9) with 8 level-2 domains, 28.1 / 29.1 (33.9 / 34.9)
+    // with 10, 24.1 / 26.5 (27.6 / 29.9) with 11, 37.6 / 33.3 (46.9 / 42.2) with 18,
+    // 51.7 / 52.0 (61.5 / 61.3) with 20, 47.6 / 47.4 (57.7 / 57.5) with 23.
     // The other CTAs share the rest, a warp a domain, when there are enough.
     const uint32_t n3 = !WIDE && M.levels > 3 ? M.num_domains - S.t.level_domain[3] : 0;
     const uint32_t n2 = WIDE ? 0 : whole - n3, nb2 = n2 > kLoopGroup ? (n2 + 2) / 3 : n2;

@@ -142,10 +142,12 @@ def main():
   def pcg_without_stream():
     keep = bs.stream
     bs.stream = False
+    mas.one_kernel_loop = False  # (small systems would take the one-kernel loop, which reads the row plan)
     try:
       mas._run_pcg(H, H.gradient.value, z, True, L.YS_PREC_MAS, None, mas._mas, 1e-30, 50, True, "residual")
     finally:
       bs.stream = keep
+      mas.one_kernel_loop = True
 
   cases = {
       "snh_eval_only": lambda: snh_eval(0),
