@@ -6,29 +6,47 @@ import threading
 import numpy as np
 import pytest
 
+from tests import test_gpu_long_rows as long_rows
 from yasps_b200 import _lib as L
 from yasps_b200 import scenes
 
 pytestmark = pytest.mark.gpu
 
 
-def make(side, mixed, seed):
+def make(side, mixed, seed, **options):
   import torch
   stream = torch.cuda.Stream()
   with torch.cuda.stream(stream):
     sc, _ = scenes.fem_scene(scenes.fem_cube(side, noise=0.01, seed=seed))
-    solver = sc.minimizer.setSolver("mas", mixed_spmv=mixed, stop_rule="residual")
-    x = sc.minimizeEnergy(tolerance=1e-6, maxIterations=500)[0].clone()
+    solver = sc.minimizer.setSolver("mas", mixed_spmv=mixed, stop_rule="residual", **options)
+    x = sc.minimizeEnergy(tolerance=1e-6, maxIterations=2000)[0].clone()
   stream.synchronize()
   return stream, sc, solver, x
 
 
-# one domain, a domain a CTA (tens of CTAs; the whole chip), warps over many domains
+def make_two_sets(side, mixed):
+  """A second block set with a row of several segments."""
+  import torch
+  stream = torch.cuda.Stream()
+  with torch.cuda.stream(stream):
+    s = long_rows.Scene(side, mixed)
+    x = s.solve(s.compute(s.hub(11))).clone()
+  stream.synchronize()
+  return stream, s, s.solver, x
+
+
+# one domain, a domain a CTA (tens of CTAs; the whole chip), warps over many
+# domains, one level, two block sets
 @pytest.mark.parametrize("mixed", [True, False])
-@pytest.mark.parametrize("side", [3, 9, 16, 25])
-def test_solution_does_not_depend_on_solves_in_flight(side, mixed):
+@pytest.mark.parametrize("side,form", [(3, "levels"), (9, "levels"), (16, "levels"), (25, "levels"),
+                                       (17, "one level"), (25, "one level"), (14, "two sets"), (72, "two sets")])
+def test_solution_does_not_depend_on_solves_in_flight(side, form, mixed):
   """Launched without waiting in between, so 1, 2, 3, 4 and 5 are in flight."""
-  solves = [make(side, mixed, 1) for _ in range(5)]
+  if form == "two sets":
+    solves = [make_two_sets(side, mixed) for _ in range(5)]
+  else:
+    options = dict(max_levels=1, global_coarse_domain=False) if form == "one level" else {}
+    solves = [make(side, mixed, 1, **options) for _ in range(5)]
   handles = [s[2].implementation._cache.handle for s in solves]
   work = [s[2].implementation for s in solves]
   before = []
