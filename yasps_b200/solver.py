@@ -39,9 +39,12 @@ class _PcgCache:
 
   def get(self, key, build):
     if key != self.key:
+      # the new handle before the old one goes: where theirs are the process's
+      # only pinned blocks, giving the last one back and making a first one
+      # again takes the driver 1.5 to 4 ms
+      handle, keepalive = build()
       self.release()
-      self.handle, self.keepalive = build()
-      self.key = key
+      self.handle, self.key, self.keepalive = handle, key, keepalive
     return self.handle
 
   def release(self):
@@ -382,8 +385,7 @@ class masSolver(_PcgBase):
     h, keep = create_mas_handle(t, nv, weights, dev)
     self._mas = h
     self._dev_tables = (dev, keep)
-    self._mas_key = key
-    self._cache.release()
+    self._mas_key = key  # (the old MAS handle is part of the PCG handle's key: the next solve makes a new one)
 
   def numeric_update(self, H, check=True):
     failed = ctypes.c_int32(0)
