@@ -992,8 +992,8 @@ cudaError_t mas_plan_loop(void* mas, int fp32, MasLoopPlan* loop) {
   return cudaSuccess;
 }
 
-cudaError_t mas_add_loop_nodes(void* mas, cudaGraph_t g, const cudaGraph_t* bodies, cudaGraphNode_t* tables,
-                               MasPcgHooks* hooks) {
+cudaError_t mas_add_loop_nodes(void* mas, cudaGraph_t g, const cudaGraph_t* bodies, int first, int count,
+                               cudaGraphNode_t* tables, MasPcgHooks* hooks) {
   const MasDev& M = static_cast<MasHandle*>(mas)->M;
   auto* P = static_cast<MasPcg*>(hooks->params);
   const MasLoopPlan& loop = hooks->loop;
@@ -1015,10 +1015,10 @@ cudaError_t mas_add_loop_nodes(void* mas, cudaGraph_t g, const cudaGraph_t* bodi
   loop_memory(L, P->nv, hooks->loop_workspace);
   void* args[] = {&L};
   cudaError_t e = add_kernel(g, tables, nullptr, 0, (const void*)loop_tables_kernel, 1, kTableThreads, 0, args);
-  for (int b = 0; b < loop.bodies && e == cudaSuccess; ++b) {
+  for (int b = first; b < first + count && e == cudaSuccess; ++b) {
     cudaGraphNode_t node = nullptr;
     const void* kernel = loop.grid[b] == loop.blocks ? loop.kernel : loop.shared_kernel;
-    e = add_kernel(bodies[b], &node, nullptr, 0, kernel, loop.grid[b], kLoopThreads, loop.smem, args);
+    e = add_kernel(bodies[b - first], &node, nullptr, 0, kernel, loop.grid[b], kLoopThreads, loop.smem, args);
     cudaKernelNodeAttrValue cv{};
     cv.cooperative = 1;
     if (e == cudaSuccess) e = cudaGraphKernelNodeSetAttribute(node, cudaKernelNodeAttributeCooperative, &cv);

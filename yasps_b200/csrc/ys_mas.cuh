@@ -6,7 +6,7 @@
 namespace ys {
 
 // Launches of the one-kernel loop (mas_pcg_loop) of one solver.  Its sums are
-// split among `blocks` virtual CTAs; body b of the solve's switch node runs
+// split among `blocks` virtual CTAs; body b of the solve's switch nodes runs
 // them on grid[b] CTAs, and body_of[k - 1] is the body while k solves of the
 // process (kLoopShares or more for the last) share the chip.
 constexpr int kLoopShares = 4;
@@ -46,10 +46,11 @@ cudaError_t mas_add_update_nodes(void* mas, cudaGraph_t body, const cudaGraphNod
 // cooperative kernel (loop->used), and its grids.
 cudaError_t mas_plan_loop(void* mas, int fp32, MasLoopPlan* loop);
 
-// That kernel as the only node of each of the loop.bodies bodies.  *tables is
-// the node of `g` that reads the row plan for it: the loop has to come after it.
-cudaError_t mas_add_loop_nodes(void* mas, cudaGraph_t g, const cudaGraph_t* bodies, cudaGraphNode_t* tables,
-                               MasPcgHooks* hooks);
+// That kernel as the only node of each of `count` bodies, on the grids from
+// loop.grid[first] on.  *tables is the node of `g` that reads the row plan for
+// it: the loop has to come after it.
+cudaError_t mas_add_loop_nodes(void* mas, cudaGraph_t g, const cudaGraph_t* bodies, int first, int count,
+                               cudaGraphNode_t* tables, MasPcgHooks* hooks);
 
 // Doubles of the solve's workspace that the one-kernel loop takes (0 beyond its sizes).
 uint64_t mas_loop_workspace_doubles(uint32_t num_vars);

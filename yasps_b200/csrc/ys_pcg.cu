@@ -442,6 +442,11 @@ struct PcgHandle {
   double params[3] = {0.0, 0.0, (double)kDefaultPollLimit};
   int device = 0;
   bool in_flight = false;  // counted in g_flight
+  // the one-kernel MAS loop on fewer CTAs, made when it is first wanted (a
+  // solver by itself is spared 0.16 ms a body)
+  void* mas_handle = nullptr;
+  cudaGraph_t shared_graph = nullptr;
+  cudaGraphExec_t shared_exec = nullptr;
 };
 
 // One-kernel MAS solves launched and not yet waited for, a count a device, and
@@ -490,6 +495,51 @@ static cudaError_t add_kernel(cudaGraph_t g, cudaGraphNode_t* node, const cudaGr
   kp.kernelParams = args;
   kp.extra = nullptr;
   return cudaGraphAddKernelNode(node, g, deps, ndeps, &kp);
+}
+
+static cudaError_t add_reset(cudaGraph_t g, cudaGraphNode_t* node, unsigned* tickets) {
+  cudaMemsetParams mp{};
+  mp.dst = tickets;
+  mp.value = 0;
+  mp.pitch = 0;
+  mp.elementSize = 4;
+  mp.width = 8;
+  mp.height = 1;
+  return cudaGraphAddMemsetNode(node, g, nullptr, 0, &mp);
+}
+
+static cudaError_t add_mas_init(PcgHandle* h, cudaGraph_t g, const cudaGraphNode_t* reset, cudaGraphNode_t* init,
+                                cudaGraphConditionalHandle cond) {
+  PcgParams& P = h->P;
+  return mas_add_init_nodes(h->mas_handle, g, reset, 1, init, P.nv, P.rhs, P.x, P.r, P.p, P.p32, P.q, P.z, P.st,
+                            P.partials, P.tickets, P.sets, P.nsets, P.fp32, P.stop_rule, P.zero_guess, P.tolerance,
+                            P.max_it, cond, &h->mas);
+}
+
+// The solve as the first residual, the loop's tables and a switch node over the
+// one-kernel loop's bodies first .. first + count - 1.
+static cudaError_t one_kernel_graph(PcgHandle* h, int first, int count, cudaGraph_t* g, cudaGraphExec_t* exec) {
+  cudaGraphConditionalHandle cond{};
+  cudaGraphNode_t reset = nullptr, init = nullptr, loop = nullptr, tables = nullptr;
+  cudaError_t e = cudaGraphCreate(g, 0);
+  if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&cond, *g, 0, cudaGraphCondAssignDefault);
+  if (e == cudaSuccess) e = add_reset(*g, &reset, h->P.tickets);
+  if (e == cudaSuccess) e = add_mas_init(h, *g, &reset, &init, cond);
+  cudaGraphNodeParams cp{};
+  cp.type = cudaGraphNodeTypeConditional;
+  cp.conditional.handle = cond;
+  cp.conditional.type = cudaGraphCondTypeSwitch;
+  cp.conditional.size = (unsigned)count;
+  if (e == cudaSuccess) e = cudaGraphAddNode(&loop, *g, &init, 1, &cp);
+  if (e == cudaSuccess) e = mas_add_loop_nodes(h->mas_handle, *g, cp.conditional.phGraph_out, first, count, &tables, &h->mas);
+  if (e == cudaSuccess) e = cudaGraphAddDependencies(*g, &tables, &loop, 1);
+  // per-node priorities (the MAS coarse chain) take effect only with this flag
+  if (e == cudaSuccess) e = cudaGraphInstantiate(exec, *g, cudaGraphInstantiateFlagUseNodePriority);
+  if (e == cudaSuccess) return e;
+  if (*g) cudaGraphDestroy(*g);
+  *g = nullptr;
+  *exec = nullptr;
+  return e;
 }
 
 }  // namespace ys
@@ -606,80 +656,69 @@ static int32_t pcg_create(const ys_pcg_args* args, bool one_kernel, void** handl
   h->params[0] = a.tolerance;
   h->params[1] = (double)a.max_iterations;
   h->preconditioner = a.preconditioner;
+  h->mas_handle = a.mas;
 
   cudaError_t e = cudaGetDevice(&h->device);
   if (e == cudaSuccess && one_kernel && a.preconditioner == YS_PREC_MAS)
     e = ys::mas_plan_loop(a.mas, P.fp32, &h->mas.loop);
   const ys::MasLoopPlan& one = h->mas.loop;
-  if (e == cudaSuccess) e = cudaGraphCreate(&h->graph, 0);
-  if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&P.cond, h->graph, 0, cudaGraphCondAssignDefault);
   if (e == cudaSuccess) e = cudaMallocHost(&h->slots_host, sizeof(double) * ys::kSlots);
-  cudaGraphNode_t reset = nullptr, init = nullptr, loop = nullptr;
-  if (e == cudaSuccess) {
-    cudaMemsetParams mp{};
-    mp.dst = P.tickets;
-    mp.value = 0;
-    mp.pitch = 0;
-    mp.elementSize = 4;
-    mp.width = 8;
-    mp.height = 1;
-    e = cudaGraphAddMemsetNode(&reset, h->graph, nullptr, 0, &mp);
-  }
-  if (e == cudaSuccess) {
-    if (a.preconditioner == YS_PREC_BLOCK_JACOBI) {
-      void* args0[] = {&P};
-      e = ys::add_kernel(h->graph, &init, &reset, 1,
-                         P.jgroup ? (const void*)ys::pcg_init_bjw : (const void*)ys::pcg_init_bj, grid, ys::kPcgBlock,
-                         args0);
-    } else {
-      e = ys::mas_add_init_nodes(a.mas, h->graph, &reset, 1, &init, P.nv, P.rhs, P.x, P.r, P.p, P.p32, P.q, P.z, P.st, P.partials,
-                                 P.tickets, P.sets, P.nsets, P.fp32, P.stop_rule, P.zero_guess, P.tolerance, P.max_it,
-                                 P.cond, &h->mas);
-    }
-  }
-  if (e == cudaSuccess) {
-    cudaGraphNodeParams cp{};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = P.cond;
-    // the one-kernel loop: a body for each grid it may run on
-    cp.conditional.type = one.used ? cudaGraphCondTypeSwitch : cudaGraphCondTypeWhile;
-    cp.conditional.size = one.used ? (unsigned)one.bodies : 1u;
-    e = cudaGraphAddNode(&loop, h->graph, &init, 1, &cp);
+  if (e == cudaSuccess && one.used) {
+    e = ys::one_kernel_graph(h, 0, 1, &h->graph, &h->exec);
+  } else if (e == cudaSuccess) {
+    e = cudaGraphCreate(&h->graph, 0);
+    if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&P.cond, h->graph, 0, cudaGraphCondAssignDefault);
+    cudaGraphNode_t reset = nullptr, init = nullptr, loop = nullptr;
+    if (e == cudaSuccess) e = ys::add_reset(h->graph, &reset, P.tickets);
     if (e == cudaSuccess) {
-      cudaGraph_t body = cp.conditional.phGraph_out[0];
-      cudaGraphNode_t n1 = nullptr, n2 = nullptr, n3 = nullptr;
-      void* args1[] = {&P};
-      if (one.used) {  // one kernel runs every iteration
-        cudaGraphNode_t tables = nullptr;
-        e = ys::mas_add_loop_nodes(a.mas, h->graph, cp.conditional.phGraph_out, &tables, &h->mas);
-        if (e == cudaSuccess) e = cudaGraphAddDependencies(h->graph, &tables, &loop, 1);
-      } else if (streamed)
-        e = ys::add_kernel(body, &n1, nullptr, 0, (const void*)ys::pcg_spmv_dot_streamed, grid_tiles,
-                           ys::kTileThreads, args1, tile_smem);
-      else if (tiled)
-        e = ys::add_kernel(body, &n1, nullptr, 0, (const void*)ys::pcg_spmv_dot_tiled, grid_tiles, ys::kTileThreads,
-                           args1, tile_smem);
-      else
-        e = ys::add_kernel(body, &n1, nullptr, 0,
-                           P.fp32 ? (const void*)ys::pcg_spmv_dot<true> : (const void*)ys::pcg_spmv_dot<false>,
-                           grid_rows, ys::kPcgBlock, args1);
-      if (e == cudaSuccess && !one.used) {
-        if (a.preconditioner == YS_PREC_BLOCK_JACOBI) {
-          e = ys::add_kernel(body, &n2, &n1, 1,
-                             P.jgroup ? (const void*)ys::pcg_update_bjw : (const void*)ys::pcg_update_bj, grid,
-                             ys::kPcgBlock, args1);
-        } else {
-          e = ys::mas_add_update_nodes(a.mas, body, &n1, 1, &n2, &h->mas);
-        }
+      if (a.preconditioner == YS_PREC_BLOCK_JACOBI) {
+        void* args0[] = {&P};
+        e = ys::add_kernel(h->graph, &init, &reset, 1,
+                           P.jgroup ? (const void*)ys::pcg_init_bjw : (const void*)ys::pcg_init_bj, grid,
+                           ys::kPcgBlock, args0);
+      } else {
+        e = ys::add_mas_init(h, h->graph, &reset, &init, P.cond);
       }
-      if (one.used || (e == cudaSuccess && a.preconditioner != YS_PREC_BLOCK_JACOBI && h->mas.fused_direction))
-        n3 = n2;  // the MAS collect kernel updated p already
-      else if (e == cudaSuccess)
-        e = ys::add_kernel(body, &n3, &n2, 1, (const void*)ys::pcg_direction, grid, ys::kPcgBlock, args1);
     }
+    if (e == cudaSuccess) {
+      cudaGraphNodeParams cp{};
+      cp.type = cudaGraphNodeTypeConditional;
+      cp.conditional.handle = P.cond;
+      cp.conditional.type = cudaGraphCondTypeWhile;
+      cp.conditional.size = 1;
+      e = cudaGraphAddNode(&loop, h->graph, &init, 1, &cp);
+      if (e == cudaSuccess) {
+        cudaGraph_t body = cp.conditional.phGraph_out[0];
+        cudaGraphNode_t n1 = nullptr, n2 = nullptr, n3 = nullptr;
+        void* args1[] = {&P};
+        if (streamed)
+          e = ys::add_kernel(body, &n1, nullptr, 0, (const void*)ys::pcg_spmv_dot_streamed, grid_tiles,
+                             ys::kTileThreads, args1, tile_smem);
+        else if (tiled)
+          e = ys::add_kernel(body, &n1, nullptr, 0, (const void*)ys::pcg_spmv_dot_tiled, grid_tiles, ys::kTileThreads,
+                             args1, tile_smem);
+        else
+          e = ys::add_kernel(body, &n1, nullptr, 0,
+                             P.fp32 ? (const void*)ys::pcg_spmv_dot<true> : (const void*)ys::pcg_spmv_dot<false>,
+                             grid_rows, ys::kPcgBlock, args1);
+        if (e == cudaSuccess) {
+          if (a.preconditioner == YS_PREC_BLOCK_JACOBI) {
+            e = ys::add_kernel(body, &n2, &n1, 1,
+                               P.jgroup ? (const void*)ys::pcg_update_bjw : (const void*)ys::pcg_update_bj, grid,
+                               ys::kPcgBlock, args1);
+          } else {
+            e = ys::mas_add_update_nodes(a.mas, body, &n1, 1, &n2, &h->mas);
+          }
+        }
+        if (e == cudaSuccess && a.preconditioner != YS_PREC_BLOCK_JACOBI && h->mas.fused_direction)
+          n3 = n2;  // the MAS collect kernel updated p already
+        else if (e == cudaSuccess)
+          e = ys::add_kernel(body, &n3, &n2, 1, (const void*)ys::pcg_direction, grid, ys::kPcgBlock, args1);
+      }
+    }
+    // per-node priorities (the MAS coarse chain) take effect only with this flag
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&h->exec, h->graph, cudaGraphInstantiateFlagUseNodePriority);
   }
-  // per-node priorities (the MAS coarse chain) take effect only with this flag
-  if (e == cudaSuccess) e = cudaGraphInstantiate(&h->exec, h->graph, cudaGraphInstantiateFlagUseNodePriority);
   if (e != cudaSuccess) {
     ys_set_last_error(cudaGetErrorString(e), __FILE__, __LINE__);
     if (h->exec) cudaGraphExecDestroy(h->exec);
@@ -703,11 +742,23 @@ int32_t ys_pcg_launch(void* handle, void* stream) {
   // parameters may change for the next launch right away.
   const ys::MasLoopPlan& one = h->mas.loop;
   int body = 0;
-  if (one.used) body = one.body_of[ys::enter_flight(h) - 1];
+  cudaGraphExec_t exec = h->exec;  // the first body; the others are in shared_exec
+  if (one.used) {
+    body = one.body_of[ys::enter_flight(h) - 1];
+    if (body > 0 && !h->shared_exec &&
+        ys::one_kernel_graph(h, 1, one.bodies - 1, &h->shared_graph, &h->shared_exec) != cudaSuccess)
+      (void)cudaGetLastError();  // the whole chip does as well
+    if (body > 0 && h->shared_exec) {
+      exec = h->shared_exec;
+      body -= 1;
+    } else {
+      body = 0;
+    }
+  }
   const double params[4] = {h->params[0], h->params[1], h->params[2], (double)body};
   cudaError_t e = cudaMemcpyAsync(h->P.st + ys::kTolParam, params, sizeof(params), cudaMemcpyHostToDevice,
                                   (cudaStream_t)stream);
-  if (e == cudaSuccess) e = cudaGraphLaunch(h->exec, (cudaStream_t)stream);
+  if (e == cudaSuccess) e = cudaGraphLaunch(exec, (cudaStream_t)stream);
   if (e != cudaSuccess) ys::leave_flight(h);
   YS_CUDA_TRY(e);
   return YS_OK;
@@ -816,6 +867,8 @@ int32_t ys_pcg_destroy(void* handle) {
   if (!handle) return YS_OK;
   auto* h = static_cast<ys::PcgHandle*>(handle);
   ys::leave_flight(h);
+  if (h->shared_exec) cudaGraphExecDestroy(h->shared_exec);
+  if (h->shared_graph) cudaGraphDestroy(h->shared_graph);
   if (h->exec) cudaGraphExecDestroy(h->exec);
   if (h->graph) cudaGraphDestroy(h->graph);
   if (h->slots_host) cudaFreeHost(h->slots_host);
